@@ -289,7 +289,8 @@ int rg_matrix_create(rg_domain* dom, rg_matrix** out)
         }
     }
     cudaError_t e = cudaSuccess;
-    if (!m.val) e = cudaMalloc((void**)&m.val, sizeof(double) * dom->d.nnz);
+    // (two more entries: bulk copies of a run of values round its end up to 16 bytes)
+    if (!m.val) e = cudaMalloc((void**)&m.val, sizeof(double) * (dom->d.nnz + 2));
     if (e == cudaSuccess && !m.bv) e = cudaMalloc((void**)&m.bv, sizeof(double) * dom->d.n);
     if (e == cudaSuccess) e = cudaMemsetAsync(m.val, 0, sizeof(double) * dom->d.nnz, stream());
     if (e != cudaSuccess) {

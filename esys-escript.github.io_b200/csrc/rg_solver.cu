@@ -13,11 +13,12 @@
 //    One FP32 iteration is one kernel (k_f32_cg, the one-reduction recurrence of
 //    Chronopoulos and Gear).
 //
-// One FP64 PCG iteration is three kernels: a pure SpMV of the search direction with its
-// p.q reduction, an elementwise update with the iteration's reductions, and an
-// elementwise kernel that forms the next search direction (in paso mode it also does
-// the smoothing step).  Scalars (alpha, beta, tau, ...) live in device memory: the last
-// CTA of each reduction kernel finishes the sum in a fixed order, sets the next step's
+// FP64 PCG runs in one persistent kernel over many iterations (rg_pcg64.cuh).  With more than
+// one Jacobi sweep (paso mode) an iteration is a kernel per step instead: a pure SpMV of the
+// search direction with its p.q reduction, an elementwise update with the iteration's
+// reductions, the extra sweeps, and an elementwise kernel that does the smoothing step and
+// forms the next search direction.  Scalars (alpha, beta, tau, ...) live in device memory: the
+// last CTA of each reduction kernel finishes the sum in a fixed order, sets the next step's
 // scalars and a `done` flag, so the host polls `done` once per chunk of iterations and
 // kernels queued after convergence return at once.  Elementwise kernels use 16-byte
 // vector accesses; matrix data is loaded with streaming (evict-first) hints so that the
@@ -25,10 +26,12 @@
 #include <chrono>
 #include <cmath>
 #include <cstdio>
+#include <algorithm>
 #include <mutex>
 #include <vector>
 
 #include "rg_bulk.cuh"
+#include "rg_gridmail.cuh"
 #include "rg_internal.cuh"
 
 namespace rg {
@@ -51,6 +54,7 @@ struct Scal {
     double best;               // FP32 path: smallest recursive residual norm of the segment
     int since;                 // iterations since `best` last dropped by 5%
     int done, status;
+    int pend, par;             // persistent FP64 PCG: an iteration's second half is done; buffer of p
 };
 
 enum { ST_RUN = 0, ST_CONV = 1, ST_MAXIT = 3, ST_BREAK = 4 };
@@ -61,6 +65,8 @@ struct Workspace {
     int64_t n = 0;
     double *r = nullptr, *x = nullptr, *rs = nullptr, *x2 = nullptr, *q = nullptr, *z = nullptr;
     double* p = nullptr;
+    double* p2 = nullptr;  // the persistent FP64 PCG's second buffer of p
+    unsigned long long* mail = nullptr;  // its grid-wide sums (rg_gridmail.cuh)
     double* bb = nullptr;  // balanced rhs
     float* d32 = nullptr;                // FP32 path: correction accumulated over a segment
     float4* v4[2] = {nullptr, nullptr};  // FP32 iteration state {u, D^-1 A u, D^-1 A p_prev, p_prev}
@@ -83,7 +89,7 @@ struct Workspace {
     bool graph_coef[3] = {false, false, false};  // the captured FP32 iterations' operator
     long long graph_launches[3][T_COUNT] = {};
     int sweeps = 1;  // Jacobi sweeps of the current paso solve (Smoother.cpp:100-128)
-    bool band64 = false;              // paso FP64 SpMV on the FP64 band copy (RG_LAYOUT_BAND)
+    bool band64 = false;              // paso FP64 with extra sweeps on the FP64 band copy (RG_LAYOUT_BAND)
     bool graph_band64[3] = {false, false, false};
     int spmv_cfg = -1;   // FP32 iteration pipeline of the band operator (kSpmvCfg; -1: not tuned)
     int coef_cfg = -1;   // the same for the element-coefficient operator (kCoefCfg)
@@ -329,6 +335,8 @@ __global__ void __launch_bounds__(kThreads) k_paso_init(int64_t n, const double*
         s->done = 0;
         s->status = ST_RUN;
         s->norm = 0.0;
+        s->pend = 0;
+        s->par = 0;
     }
 }
 
@@ -529,105 +537,11 @@ __global__ void __launch_bounds__(kThreads) k_std_init(int64_t n, const double* 
         s->maxit = maxit;
         s->tol = tol;
         s->status = ST_RUN;
+        s->pend = 0;
+        s->par = 0;
         s->done = (s->norm <= tol) ? 1 : 0;
         if (s->done) s->status = ST_CONV;
     }
-}
-
-__global__ void __launch_bounds__(kThreads) k_std_spmv(int64_t n, const int32_t* __restrict__ ptr,
-                                                       const int32_t* __restrict__ idx,
-                                                       const double* __restrict__ val,
-                                                       const double* __restrict__ p,
-                                                       double* __restrict__ q, ReduceBuf rb, Scal* s)
-{
-    if (s->done) return;
-    double v[1] = {0.0};
-    RG_ROW_LOOP(n)
-    {
-        double acc = row < n ? csr_row_dot(ptr, idx, val, p, row, lane) : 0.0;
-        acc = group_sum(acc);
-        if (row < n && lane == 0) {
-            q[row] = acc;
-            v[0] += acc * p[row];
-        }
-    }
-    double t[1];
-    if (grid_reduce<1>(v, rb, t) && threadIdx.x == 0) {
-        s->delta = t[0];
-        s->alpha = s->rho / t[0];
-        if (!(fabs(t[0]) > 0.0)) {
-            s->iter += 1;
-            s->status = ST_BREAK;
-            s->done = 1;
-        }
-    }
-}
-
-// x += alpha p; r -= alpha q; z = dinv r; rho_next = r.z, ||r||^2; stopping tests; beta
-__global__ void __launch_bounds__(kThreads) k_std_update(int64_t n, double* __restrict__ x,
-                                                         double* __restrict__ r,
-                                                         const double* __restrict__ q,
-                                                         const double* __restrict__ p,
-                                                         const double* __restrict__ dinv,
-                                                         double* __restrict__ z, ReduceBuf rb, Scal* s)
-{
-    if (s->done) return;
-    const double alpha = s->alpha;
-    double v[2] = {0.0, 0.0};
-    const int64_t nv = n >> 1;
-    for (int64_t k = gtid(); k < nv; k += gstride()) {
-        const double2 x0 = ld2(x, k), r0 = ld2(r, k), q0 = ld2(q, k), p0 = ld2(p, k), di = ld2(dinv, k);
-        st2(x, k, make_double2(x0.x + alpha * p0.x, x0.y + alpha * p0.y));
-        const double ra = r0.x - alpha * q0.x, rb2 = r0.y - alpha * q0.y;
-        st2(r, k, make_double2(ra, rb2));
-        const double za = ra * di.x, zb = rb2 * di.y;
-        st2(z, k, make_double2(za, zb));
-        v[0] += za * ra + zb * rb2;
-        v[1] += ra * ra + rb2 * rb2;
-    }
-    if ((n & 1) && gtid() == 0) {
-        const int64_t i = n - 1;
-        x[i] += alpha * p[i];
-        const double ri = r[i] - alpha * q[i];
-        r[i] = ri;
-        const double zi = ri * dinv[i];
-        z[i] = zi;
-        v[0] += zi * ri;
-        v[1] += ri * ri;
-    }
-    double t[2];
-    if (grid_reduce<2>(v, rb, t) && threadIdx.x == 0) {
-        const long long it = s->iter + 1;
-        s->iter = it;
-        const double norm = sqrt(t[1]);
-        s->norm = norm;
-        s->beta = t[0] / s->rho;
-        const bool brk = !(fabs(t[0]) > 0.0);
-        s->rho = t[0];
-        if (norm <= s->tol) {
-            s->status = ST_CONV;
-            s->done = 1;
-        } else if (it >= s->maxit) {
-            s->status = ST_MAXIT;
-            s->done = 1;
-        } else if (brk) {
-            s->status = ST_BREAK;
-            s->done = 1;
-        }
-    }
-}
-
-__global__ void __launch_bounds__(kThreads) k_std_pupdate(int64_t n, const double* __restrict__ z,
-                                                          double* __restrict__ p, const Scal* s)
-{
-    if (s->done) return;
-    const double beta = s->beta;
-    const int64_t nv = n >> 1;
-    for (int64_t k = gtid(); k < nv; k += gstride()) {
-        const double2 z0 = ld2(z, k), p0 = ld2(p, k);
-        st2(p, k, make_double2(z0.x + beta * p0.x, z0.y + beta * p0.y));
-    }
-    if ((n & 1) && gtid() == 0) p[n - 1] = z[n - 1] + beta * p[n - 1];
 }
 
 // ------------------------------------------------------------------ FP32 PCG on the band copy
@@ -691,15 +605,14 @@ __global__ void __launch_bounds__(kThreads) k_cheb_step_band(const __grid_consta
     }
 }
 
-// The FP64 band kernels of the paso PCG (RG_LAYOUT_BAND), warp-specialised and persistent
+// The FP64 band kernels of the paso PCG with extra sweeps (RG_LAYOUT_BAND), warp-specialised and persistent
 // like k_f32_cg: lane 0 of warp kConsumerWarps streams, per tile, the tile's FP64 band
 // block (one bulk copy, L2 evict-first) and, for interior tiles, the NG windows of x its
 // stencil columns span (kTile+4 values from a 16-byte aligned start) into a kStages ring;
 // consumer warps compute row i0 + t from shared memory.  Tiles near the two ends read x with
 // clamped loads.  The bands are summed in column order.
-//   SWEEP = false: v = A x, delta = x.v; mode 0: alpha = tau/delta, breakdown on delta == 0
-//                  (PCG.cpp:223-262), i.e. k_paso_spmv; mode 1: alpha = rho/delta, i.e.
-//                  k_std_spmv (RG_MODE_STANDARD).
+//   SWEEP = false: v = A x, delta = x.v, alpha = tau/delta, breakdown on delta == 0
+//                  (PCG.cpp:223-262), i.e. k_paso_spmv.
 //   SWEEP = true:  one Jacobi sweep out = x + dinv (b - A x) with k_jacobi_sweep's modes.
 // All waits are bounded: on timeout the kernel records ST_TIMEOUT and returns.
 constexpr int kWin64 = kTile + 4;
@@ -835,17 +748,10 @@ __global__ void __launch_bounds__(kTile + 32, 1) k_band64_bulk(const double* __r
     if (SWEEP && mode == 0) return;
     double tt[1];
     if (grid_reduce<1>(v, rb, tt) && threadIdx.x == 0) {
-        if (!SWEEP && mode == 0) {
+        if (!SWEEP) {
             s->delta = tt[0];
             s->alpha = s->tau / tt[0];
             if (fabs(tt[0]) <= 0.0) {  // breakFlag
-                s->iter += 1;
-                report_status(s, ST_BREAK);
-            }
-        } else if (!SWEEP) {
-            s->delta = tt[0];
-            s->alpha = s->rho / tt[0];
-            if (!(fabs(tt[0]) > 0.0)) {
                 s->iter += 1;
                 report_status(s, ST_BREAK);
             }
@@ -861,6 +767,8 @@ __global__ void __launch_bounds__(kTile + 32, 1) k_band64_bulk(const double* __r
 // stages of the FP64 band ring: 3 x 74 KB (27 bands) or 8 x 24 KB (9 bands), one CTA per SM
 template <int NB>
 constexpr int band64_stages() { return NB == 27 ? 3 : 8; }
+
+#include "rg_pcg64.cuh"
 
 // ------------------------------------------------------------------ FP32 PCG, one kernel per iteration
 // Jacobi-PCG in the one-reduction form of Chronopoulos and Gear ("s-step iterative methods
@@ -1547,7 +1455,7 @@ void launch_band64(Matrix* m, const double* x, double* out, const double* b, dou
     const TmaBandArgs ta = band_offsets(d);
     const int64_t ntiles = (d->n + kTile - 1) / kTile;
     const int grid = (int)std::min<int64_t>(ntiles, sm_count());
-    const int kind = SWEEP ? T_PASO_UPDATE1 : (mode == 1 ? T_STD_SPMV : T_PASO_SPMV);
+    const int kind = SWEEP ? T_PASO_UPDATE1 : T_PASO_SPMV;
     if (d->nbands == 27) {
         constexpr int S = band64_stages<27>();
         RG_TIMED(kind, (k_band64_bulk<27, S, SWEEP><<<grid, kTile + 32, band64_smem<27, S>(), stream()>>>(
@@ -1598,22 +1506,6 @@ int paso_step(Matrix* m)
     return RG_OK;
 }
 
-int std_step(Matrix* m)
-{
-    Workspace* w = m->ws;
-    const Domain* d = m->dom;
-    if (w->band64 && m->band64)
-        launch_band64<false>(m, w->p, w->q, nullptr, nullptr, 1);
-    else
-        RG_TIMED(T_STD_SPMV, (k_std_spmv<<<w->grid_rows, kThreads, 0, stream()>>>(d->n, d->ptr, d->idx, m->val,
-                                                                                  w->p, w->q, rbuf(w), w->s)));
-    RG_TIMED(T_STD_UPDATE, (k_std_update<<<w->grid_vec, kThreads, 0, stream()>>>(d->n, w->x, w->r, w->q, w->p,
-                                                                                 m->dinv, w->z, rbuf(w), w->s)));
-    RG_TIMED(T_VECTOR, (k_std_pupdate<<<w->grid_vec, kThreads, 0, stream()>>>(d->n, w->z, w->p, w->s)));
-    RG_CHECK_LAUNCH();
-    return RG_OK;
-}
-
 int sm_count()
 {
     static int count = 0;
@@ -1624,6 +1516,90 @@ int sm_count()
         if (count <= 0) count = kNumSMs;
     }
     return count;
+}
+
+// warps and ring stages of k_pcg64: 16 warps x 2 x 6.9 KB (27 bands) or 16 x 6 x 2.3 KB (9)
+constexpr int kPcgWarps = 16;
+template <int NB>
+constexpr int pcg64_stages() { return NB == 27 ? 2 : 6; }
+
+template <int NB, bool PASO>
+int run_pcg64_t(Matrix* m, long long cap, long long* iters, int* status)
+{
+    constexpr int W = kPcgWarps, S = pcg64_stages<NB>();
+    Workspace* w = m->ws;
+    const Domain* d = m->dom;
+    const int64_t n = d->n;
+    static std::once_flag once;
+    static cudaError_t attr = cudaSuccess;
+    std::call_once(once, [] {
+        attr = cudaFuncSetAttribute(k_pcg64<NB, W, S, PASO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)pcg64_smem<NB, W, S>());
+    });
+    RG_CHECK_CUDA(attr);
+    Pcg64Args a{};
+    a.n = (int)n;
+    a.nn0 = (int)d->nn[0];
+    a.nn1 = (int)d->nn[1];
+    a.nn2 = (int)d->nn[2];
+    for (int b = 0; b < NB; ++b) a.off[b] = (int)d->band_off[b];
+    fast_div((unsigned)a.nn0, &a.m0, &a.s0);
+    fast_div((unsigned)(a.nn0 * a.nn1), &a.m1, &a.s1);
+    a.ptr = d->ptr;
+    a.val = m->val;
+    a.r = w->r;
+    a.q = w->q;
+    a.rs = w->rs;
+    a.x = w->x;
+    a.x2 = w->x2;
+    a.z = w->z;
+    a.p0 = w->p;
+    a.p1 = w->p2;
+    a.dinv = m->dinv;
+    a.mail = w->mail;
+    a.ntiles = (int)((n + 31) / 32);
+    // tiles spread evenly: rounds of the grid, then as many active warps per CTA as a round needs
+    // (with few rounds a last, nearly empty one would cost as much as a full one)
+    const int sms = std::min(sm_count(), kMailCtas);
+    const int64_t rounds = (a.ntiles + (int64_t)sms * W - 1) / ((int64_t)sms * W);
+    a.wpc = (int)std::min<int64_t>(W, (a.ntiles + sms * rounds - 1) / (sms * rounds));
+    const int grid = (int)std::min<int64_t>(sms, (a.ntiles + a.wpc - 1) / a.wpc);
+    // about 20 ms of iterations per launch
+    const double iter_s = (double)n * (8 * NB + 140) / 5.0e12 + 5e-6;
+    a.max_iters = (int)std::min(std::max(0.02 / iter_s, 16.0), 8192.0);
+    const int kind = PASO ? T_PASO_SPMV : T_STD_SPMV;
+    long long launched = 0;
+    for (;;) {
+        RG_CHECK_CUDA(cudaMemsetAsync(w->mail, 0, kMailBytes, stream()));
+        Scal* s = w->s;
+        void* args[] = {&a, &s};
+        cudaError_t e;
+        RG_TIMED(kind, (e = cudaLaunchCooperativeKernel((const void*)k_pcg64<NB, W, S, PASO>, dim3(grid),
+                                                        dim3(W * 32), args, pcg64_smem<NB, W, S>(), stream())));
+        RG_CHECK_CUDA(e);
+        launched += a.max_iters;
+        int rc = read_scal(w);
+        if (rc) return rc;
+        if (w->hs->done) break;
+        if (launched > cap + 2LL * a.max_iters + 8) {
+            set_error("PCG iteration loop did not terminate");
+            return RG_TIMEOUT;
+        }
+    }
+    *iters = w->hs->iter;
+    *status = w->hs->status;
+    return RG_OK;
+}
+
+// FP64 PCG iterations until the device flags done (one Jacobi sweep per preconditioner)
+int run_pcg64(Matrix* m, bool paso, long long cap, long long* iters, int* status)
+{
+    Workspace* w = m->ws;
+    if (!w->p2) RG_CHECK_CUDA(cudaMalloc((void**)&w->p2, sizeof(double) * m->dom->n));
+    if (!w->mail) RG_CHECK_CUDA(cudaMalloc((void**)&w->mail, kMailBytes));
+    if (m->dom->nbands == 27)
+        return paso ? run_pcg64_t<27, true>(m, cap, iters, status) : run_pcg64_t<27, false>(m, cap, iters, status);
+    return paso ? run_pcg64_t<9, true>(m, cap, iters, status) : run_pcg64_t<9, false>(m, cap, iters, status);
 }
 
 // configurations of the FP32 iteration pipeline: (stages, CTAs per SM), for the band operator
@@ -2037,7 +2013,7 @@ int solve_fp64(Matrix* m, const rg_solver_opts* o, bool paso, OuterState& st, rg
 {
     Workspace* w = m->ws;
     const int64_t n = m->dom->n;
-    const int chunk = chunk_for(n, paso ? 12 * 27 + 160 : 12 * 27 + 112);
+    const int chunk = chunk_for(n, 12 * 27 + 160);
     bool first = true;
     for (;;) {
         const long long cnt = o->iter_max - st.totIter;
@@ -2058,12 +2034,15 @@ int solve_fp64(Matrix* m, const rg_solver_opts* o, bool paso, OuterState& st, rg
             RG_CHECK_LAUNCH();
             jacobi_sweeps(m, w->r, w->z, w->q, w->p, 2);  // the first v = prec(r): p and tau
             RG_CHECK_LAUNCH();
-            if ((rc = run_until_done(m, 0, paso_step, chunk, cnt, &it, &dst))) return rc;
+            // more than one Jacobi sweep has an SpMV inside the preconditioner: one kernel per step
+            rc = w->sweeps > 1 ? run_until_done(m, 0, paso_step, chunk, cnt, &it, &dst)
+                               : run_pcg64(m, true, cnt, &it, &dst);
+            if (rc) return rc;
         } else {
             RG_TIMED(T_VECTOR, (k_std_init<<<w->grid_rows, kThreads, 0, stream()>>>(
                                    n, w->r, m->dinv, w->z, w->p, rbuf(w), w->s, tol, cnt > 0 ? cnt : 1)));
             RG_CHECK_LAUNCH();
-            if ((rc = run_until_done(m, 1, std_step, chunk, cnt, &it, &dst))) return rc;
+            if ((rc = run_pcg64(m, false, cnt, &it, &dst))) return rc;
         }
         st.totIter += it;
         bool restart = false;
@@ -2248,8 +2227,9 @@ void free_workspace(Matrix* m)
 {
     Workspace* w = m->ws;
     if (!w) return;
-    double* dd[] = {w->r, w->x, w->rs, w->x2, w->q, w->z, w->p, w->bb, w->partials};
+    double* dd[] = {w->r, w->x, w->rs, w->x2, w->q, w->z, w->p, w->p2, w->bb, w->partials};
     for (double* p : dd) cudaFree(p);
+    cudaFree(w->mail);
     cudaFree(w->d32);
     cudaFree(w->v4[0]);
     cudaFree(w->v4[1]);
@@ -2337,7 +2317,9 @@ int solve_impl(Matrix* m, const double* rhs, double* x, const rg_solver_opts* o,
     // every grid reduction leaves the counter at zero; clearing it here as well keeps one
     // solve independent of anything an earlier, interrupted one left behind
     RG_CHECK_CUDA(cudaMemsetAsync(w->counter, 0, sizeof(unsigned), stream()));
-    const bool band64 = !fp32 && o->layout == RG_LAYOUT_BAND;
+    // the FP64 band copy serves the extra Jacobi sweeps; with one sweep the persistent PCG streams
+    // the CSR values without their column indices, the same bytes
+    const bool band64 = paso && o->sweeps > 1 && o->layout == RG_LAYOUT_BAND;
     if (!fp32 && o->layout == RG_LAYOUT_COEF) {
         set_error("solver: RG_LAYOUT_COEF evaluates the FP32 inner operator; FP64 solves use RG_LAYOUT_CSR or "
                   "RG_LAYOUT_BAND");

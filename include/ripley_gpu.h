@@ -189,10 +189,12 @@ int rg_save_mm(rg_matrix* mat, const char* path);
 #define RG_PREC_FP32_REFINE 1     /* FP32 inner PCG, FP64 residual/update/stop test         */
 #define RG_LAYOUT_CSR 0           /* inner SpMV on the paso CSR values                       */
 #define RG_LAYOUT_BAND 1          /* SpMV on a 27-band (9 in 2D) structured copy: FP32_REFINE
-                                     always; FP64 solves (paso or standard mode) with this
-                                     layout stream an FP64 band copy (8 bytes per coefficient
-                                     against the CSR's 12).  Scalar PDEs only: systems
-                                     (block size 2, 3) always use the block CSR            */
+                                     always; FP64 paso solves with extra Jacobi sweeps and
+                                     this layout stream an FP64 band copy.  FP64 solves with
+                                     one sweep run alike with either layout: they read the
+                                     CSR values without the column indices (8 bytes per
+                                     entry).  Scalar PDEs only: systems (block size 2, 3)
+                                     always use the block CSR                             */
 #define RG_LAYOUT_COEF 2          /* FP32_REFINE only: the FP32 inner PCG evaluates the operator
                                      from the element coefficients instead of streaming stored
                                      values (4 bytes per row instead of 108), when the matrix's
@@ -271,8 +273,8 @@ int rg_solver_config(const rg_matrix* mat, int* spmv_config, int* update_grid, d
 int rg_solver_set_config(rg_matrix* mat, int spmv_config);
 
 /* Test hook for the timeout path of the warp-specialised kernels (no reference counterpart;
-   paso has no device waits).  max_polls > 0 caps the polls of each bounded wait of the band
-   kernels (FP32_REFINE, and FP64 with RG_LAYOUT_BAND) and of the persistent convolution of
+   paso has no device waits).  max_polls > 0 caps the polls of each bounded wait of the
+   warp-specialised and persistent kernels (FP32_REFINE and FP64 solves) and of the persistent convolution of
    rg_ws_conv3; 0 restores the default limit.  withhold_copies != 0 makes their producers
    issue no copies, so every wait runs out with nothing in flight: a solve then returns
    RG_TIMEOUT, a convolution sets its device error flag, and the matrix, its domain and the
