@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
         fetch(mine - 1);
         double t[2];
         ++gen;
-        bool ok = mail_sum<2, W, false>(v, t, a.mail, gen, &bad, polls);
+        bool ok = mail_sum<2, W, false>(v, t, a.mail, gen, &bad, polls, wc.withhold != 0);
         if (threadIdx.x == 0) {
             if (!ok) {
                 sc.status = ST_TIMEOUT;
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
         }
         double w[3];
         ++gen;
-        ok = mail_sum<3, W, true>(u, w, a.mail, gen, &bad, polls);
+        ok = mail_sum<3, W, true>(u, w, a.mail, gen, &bad, polls, wc.withhold != 0);
         if (threadIdx.x == 0) {
             if (!ok) {
                 sc.status = ST_TIMEOUT;

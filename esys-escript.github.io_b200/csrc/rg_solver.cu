@@ -55,7 +55,11 @@ struct Scal {
     int since;                 // iterations since `best` last dropped by 5%
     int done, status;
     int pend, par;             // persistent FP64 PCG: an iteration's second half is done; buffer of p
+    double dpend;              // FP32 on the coefficients: the step length d has yet to take (dpend_on)
+    int dpend_on;
 };
+
+#include "rg_march.cuh"
 
 enum { ST_RUN = 0, ST_CONV = 1, ST_MAXIT = 3, ST_BREAK = 4 };
 
@@ -86,7 +90,6 @@ struct Workspace {
     cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};
     int graph_chunk[3] = {0, 0, 0};
     int graph_sweeps[3] = {0, 0, 0};  // Jacobi sweeps the captured iterations apply
-    bool graph_coef[3] = {false, false, false};  // the captured FP32 iterations' operator
     long long graph_launches[3][T_COUNT] = {};
     int sweeps = 1;  // Jacobi sweeps of the current paso solve (Smoother.cpp:100-128)
     bool band64 = false;              // paso FP64 with extra sweeps on the FP64 band copy (RG_LAYOUT_BAND)
@@ -133,7 +136,8 @@ int ensure_workspace(Matrix* m, bool fp32)
             (rc = dalloc(&w->x2, n)) || (rc = dalloc(&w->q, n)) || (rc = dalloc(&w->z, n)) ||
             (rc = dalloc(&w->p, n)) || (rc = dalloc(&w->bb, n)) ||
             (rc = dalloc(&w->partials, (size_t)4 * kNumSMs * 64)) || (rc = dalloc(&w->counter, 1)) ||
-            (rc = dalloc(&w->s, 1)) || (rc = dalloc(&w->bad, 1)))
+            (rc = dalloc(&w->s, 1)) || (rc = dalloc(&w->bad, 1)) ||
+            (rc = dalloc((unsigned char**)&w->mail, kMailBytes)))
             return rc;
         RG_CHECK_CUDA(cudaMallocHost((void**)&w->hs, sizeof(Scal)));
         RG_CHECK_CUDA(cudaMallocHost((void**)&w->hpoll, 2 * sizeof(Scal)));
@@ -814,10 +818,7 @@ struct CgArgs {
     int nwin, wlen;        // windows per tile and rows per window
     int64_t n;
     int64_t lo, hi;        // a tile is interior when i0 + lo >= 0 and i0 + hi <= n
-    // element-coefficient operator (RG_LAYOUT_COEF): khat windows and the Q1 table
-    int kwoff[4];          // khat window offsets (multiples of 4: 16-byte aligned starts)
-    int nkw, kwlen;        // khat windows per tile and floats per window (a multiple of 4)
-    int kpos[8];           // shared-memory float index of corner element j = a + 2b + 4c for row 0
+    // element-coefficient operator (RG_LAYOUT_COEF): the seed and the guess smoothing
     int kdelta[8];         // khat offset of corner element j: a + NN0 b + NN0 NN1 c
     float T[8];            // Q1 stiffness entry for nodes differing in x (bit 0), y (1), z (2)
 };
@@ -915,17 +916,9 @@ __device__ void cg_scalars(Scal* s, const double* tt, int mode)
     }
 }
 
-// Fused FP32 PCG iteration, two operators:
-//   COEF = false: the tile's band block (FP32 copy of the balanced matrix) is bulk-copied with
-//                 the state windows; the diagonal is its centre band.
-//   COEF = true:  the operator is evaluated from the element coefficients (unbalanced A; the
-//                 Jacobi-preconditioned iteration is the same for any symmetric diagonal scaling
-//                 of the matrix, so the balancing is applied only where the FP64 refinement
-//                 hands residuals and corrections over): windows of khat replace the band
-//                 block (4 instead of 108 bytes per row).  Rows of nodes fixed by the constraint
-//                 are identity rows, solved exactly by the seed; their state stays zero, so
-//                 their columns drop out of every other row without a mask.
-template <int NB, int kStages, int kCtas, bool COEF>
+// Fused FP32 PCG iteration on the band copy: the tile's band block (FP32 copy of the balanced matrix)
+// is bulk-copied with the state windows; the diagonal is its centre band.
+template <int NB, int kStages, int kCtas>
 __global__ void __launch_bounds__(kTile + 32, kCtas) k_f32_cg(const float* __restrict__ band,
                                                               const __grid_constant__ CgArgs ca,
                                                               const float4* V0, const float4* V1,
@@ -934,7 +927,6 @@ __global__ void __launch_bounds__(kTile + 32, kCtas) k_f32_cg(const float* __res
 {
     constexpr int kCenter = NB / 2;
     constexpr int NG = NB / 3;
-    constexpr int NK = NB == 27 ? 8 : 4;  // elements around a node
     extern __shared__ __align__(128) float smem[];
     __shared__ __align__(8) uint64_t full[kStages], empty[kStages];
     __shared__ int bad;
@@ -951,15 +943,14 @@ __global__ void __launch_bounds__(kTile + 32, kCtas) k_f32_cg(const float* __res
     const int64_t n = ca.n;
     const int64_t ntiles = (n + kTile - 1) / kTile;
     const int64_t my_tiles = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-    // tile k of this CTA; on the band operator odd iterations walk the tiles backwards, so that
-    // the state rows the previous launch wrote last, the likeliest to be still in L2, are read
-    // first (measured at 128^3: 58.4 -> 55.4 us per launch; the coefficient operator, whose
-    // launch is not bound by memory, gained nothing and spilled registers with it)
-    const bool back = !COEF && odd;
+    // tile k of this CTA; odd iterations walk the tiles backwards, so that the state rows the
+    // previous launch wrote last, the likeliest to be still in L2, are read first (measured at
+    // 128^3: 58.4 -> 55.4 us per launch)
+    const bool back = odd;
     const int64_t tbase = back ? ntiles - 1 - blockIdx.x : (int64_t)blockIdx.x;
     const int64_t tstep = back ? -(int64_t)gridDim.x : (int64_t)gridDim.x;
     auto tile_of = [&](int64_t k) { return tbase + k * tstep; };
-    const int kmat = COEF ? ca.nkw * ca.kwlen : NB * kTile;  // floats of the operator's part of a stage
+    constexpr int kmat = NB * kTile;  // floats of the operator's part of a stage
     const int stage_floats = kmat + 4 * ca.nwin * ca.wlen;
     if (t == 0) {
         for (int k = 0; k < kStages; ++k) {
@@ -993,13 +984,7 @@ __global__ void __launch_bounds__(kTile + 32, kCtas) k_f32_cg(const float* __res
                 float* dst = smem + (size_t)st * stage_floats;
                 const bool in = interior(i0);
                 mbar_expect_tx(&full[st], (uint32_t)kmat * 4u + (in ? (uint32_t)ca.nwin * wbytes : 0u));
-                if (COEF) {
-                    // khat is padded: every tile's windows are in range
-                    for (int w = 0; w < ca.nkw; ++w)
-                        bulk_g2s(dst + w * ca.kwlen, band + (i0 + ca.kwoff[w]), (uint32_t)ca.kwlen * 4u, &full[st]);
-                } else {
-                    bulk_g2s_hint(dst, band + (size_t)tile * NB * kTile, NB * kTile * 4, &full[st], pol);
-                }
+                bulk_g2s_hint(dst, band + (size_t)tile * NB * kTile, NB * kTile * 4, &full[st], pol);
                 if (in)
                     for (int w = 0; w < ca.nwin; ++w)
                         bulk_g2s(dst + kmat + 4 * w * ca.wlen, vin + (i0 + ca.woff[w]), wbytes, &full[st]);
@@ -1019,33 +1004,10 @@ __global__ void __launch_bounds__(kTile + 32, kCtas) k_f32_cg(const float* __res
             }
             const float* bs = smem + st * stage_floats;
             const float4* win = reinterpret_cast<const float4*>(bs + kmat);
-            // this row's coefficients: formed from the element values (COEF), or read from the
-            // band block where they are used
-            CoefRow cr;
-            bool fixed = false;
-            if constexpr (COEF) {
-                float kv[8];
-#pragma unroll
-                for (int j = 0; j < NK; ++j) kv[j] = bs[ca.kpos[j] + t];
-                fixed = (__float_as_uint(kv[0]) >> 31) != 0;
-#pragma unroll
-                for (int j = 0; j < NK; ++j) kv[j] = fabsf(kv[j]);
-#pragma unroll
-                for (int j = NK; j < 8; ++j) kv[j] = 0.f;
-                coef_row<NB>(kv, cr);
-            }
-            auto coefb = [&](int b) -> float {
-                if constexpr (COEF)
-                    return coef_at<NB>(cr, ca.T, b);
-                else
-                    return bs[b * kTile + t];
-            };
+            auto coefb = [&](int b) -> float { return bs[b * kTile + t]; };
             float acc_u = 0.f, acc_p = 0.f;
             float4 c = make_float4(0.f, 0.f, 0.f, 0.f);  // this row's state
             if (interior(i0) && mode == 0) {
-                // (a row's products are summed in band order: summing them per Q1 table class
-                // and scaling once was measured to cost ~7% more iterations at 128^3, from the
-                // FP32 cancellation of a Laplacian row's nearly zero sum)
 #pragma unroll
                 for (int g = 0; g < NG; ++g) {
                     // u_{i+1} at this lane's dx = 0 neighbour of stencil column g; dx = -1 / +1
@@ -1084,12 +1046,7 @@ __global__ void __launch_bounds__(kTile + 32, kCtas) k_f32_cg(const float* __res
                     if (b == kCenter) c = nb;
                 }
             }
-            float diag = coefb(kCenter);
-            if (COEF && fixed) {  // identity row: solved by the seed, state stays zero
-                acc_u = 0.f;
-                acc_p = 0.f;
-                diag = 1.f;
-            }
+            const float diag = coefb(kCenter);
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[st]);
             if (i < n) {
@@ -1108,11 +1065,7 @@ __global__ void __launch_bounds__(kTile + 32, kCtas) k_f32_cg(const float* __res
                 vout[i] = make_float4(un, __fdividef(w, diag), spn, pn);
                 const double du = un, dd = diag, ds = (double)spn * dd;
                 v[0] += dd * du * du;
-                // the segment's stopping norm: |r| of the balanced residual (band copy); for the
-                // unbalanced coefficient operator r.u = r.D^-1 r (= v[0], copied after the
-                // reduction), which paso's balancing leaves unchanged and which is |B r|^2 when
-                // the balance vector is D^-1/2 (diagonally dominant rows)
-                if (!COEF) v[1] += (dd * du) * (dd * du);
+                v[1] += (dd * du) * (dd * du);  // the segment's stopping norm: |r|^2 of the balanced residual
                 v[2] += du * (double)w;
                 v[3] += du * ds;
                 v[4] += (double)pn * (double)w;
@@ -1135,10 +1088,11 @@ __global__ void __launch_bounds__(kTile + 32, kCtas) k_f32_cg(const float* __res
     }
     double tt[6];
     if (grid_reduce<6>(v, rb, tt) && threadIdx.x == 0) {
-        if (COEF) tt[1] = tt[0];
         cg_scalars(s, tt, mode);
     }
 }
+
+#include "rg_cg_coef.cuh"
 
 // The element-coefficient operator's seed: the balanced FP64 residual is unbalanced (r =
 // r64 / bv, scaled by inv_scale); fixed nodes get their exact correction d = r (identity
@@ -1243,12 +1197,18 @@ __global__ void __launch_bounds__(kThreads) k_cheb_step_coef(const __grid_consta
     }
 }
 
-// x64 += scale * d32 / bv (the element-coefficient operator's correction is unbalanced); d32 = 0
+// x64 += scale * d32 / bv (the element-coefficient operator's correction is unbalanced), with the last
+// step d has not taken yet (s->dpend times the direction in the current state); d32 = 0
 __global__ void k_fold_correction_unbalance(int64_t n, double* __restrict__ x, float* __restrict__ d,
-                                            const double* __restrict__ bv, double scale)
+                                            const float4* V0, const float4* V1, const double* __restrict__ bv,
+                                            const Scal* s, double scale)
 {
+    const float4* v = (s->pk & 1) ? V1 : V0;
+    const bool pend = s->dpend_on != 0;
+    const float a = (float)s->dpend;
     for (int64_t i = gtid(); i < n; i += gstride()) {
-        x[i] += scale * (double)d[i] / bv[i];
+        const float di = pend ? fmaf(a, v[i].w, d[i]) : d[i];
+        x[i] += scale * (double)di / bv[i];
         d[i] = 0.f;
     }
 }
@@ -1308,6 +1268,8 @@ int write_scal_fields(Workspace* w, double tol, long long maxit, long long iter0
     h.since = 0;
     h.done = 0;
     h.status = ST_RUN;
+    h.dpend = 0.0;
+    h.dpend_on = 0;
     *w->hs = h;
     RG_CHECK_CUDA(cudaMemcpyAsync(w->s, w->hs, sizeof(Scal), cudaMemcpyHostToDevice, stream()));
     return RG_OK;
@@ -1365,7 +1327,7 @@ int run_until_done(Matrix* m, int kind, IterFn step, int chunk, long long cap, l
         return RG_OK;
     }
     if (!w->graph[kind] || w->graph_chunk[kind] != chunk || w->graph_sweeps[kind] != w->sweeps ||
-        w->graph_band64[kind] != w->band64 || w->graph_coef[kind] != w->coef_op) {
+        w->graph_band64[kind] != w->band64) {
         if (w->graph[kind]) cudaGraphExecDestroy(w->graph[kind]);
         w->graph[kind] = nullptr;
         long long before[T_COUNT], after[T_COUNT];
@@ -1389,7 +1351,6 @@ int run_until_done(Matrix* m, int kind, IterFn step, int chunk, long long cap, l
         w->graph_chunk[kind] = chunk;
         w->graph_sweeps[kind] = w->sweeps;
         w->graph_band64[kind] = w->band64;
-        w->graph_coef[kind] = w->coef_op;
         timers_snapshot(after);
         long long undo[T_COUNT];
         for (int k = 0; k < T_COUNT; ++k) {
@@ -1596,16 +1557,34 @@ int run_pcg64(Matrix* m, bool paso, long long cap, long long* iters, int* status
 {
     Workspace* w = m->ws;
     if (!w->p2) RG_CHECK_CUDA(cudaMalloc((void**)&w->p2, sizeof(double) * m->dom->n));
-    if (!w->mail) RG_CHECK_CUDA(cudaMalloc((void**)&w->mail, kMailBytes));
     if (m->dom->nbands == 27)
         return paso ? run_pcg64_t<27, true>(m, cap, iters, status) : run_pcg64_t<27, false>(m, cap, iters, status);
     return paso ? run_pcg64_t<9, true>(m, cap, iters, status) : run_pcg64_t<9, false>(m, cap, iters, status);
 }
 
-// configurations of the FP32 iteration pipeline: (stages, CTAs per SM), for the band operator
-// and for the element-coefficient operator (whose stages are a quarter of the size)
+// configurations of the FP32 iteration: (stages, CTAs per SM) of the pipeline on the band copy,
+// warps per CTA (one CTA per SM) and, in 3D, x-lines per lane on the element coefficients
 constexpr int kSpmvCfg[2][2] = {{3, 1}, {2, 2}};
-constexpr int kCoefCfg[2][2] = {{3, 2}, {2, 2}};
+constexpr int kCoefWarps[2] = {16, 28}, kCoefLines[2] = {2, 1};
+
+// Q1 stiffness of the reference box by which coordinates differ (bit 0 x, 1 y, 2 z), exact 1D
+// integrals (the 2-point Gauss rule of the assembly is exact for them): per axis K = 1/h (same
+// node) or -1/h, M = h/3 or h/6
+void q1_table(const Domain* d, double (&T)[8])
+{
+    const bool three = d->dim == 3;
+    for (int cls = 0; cls < 8; ++cls) {
+        double k1[3], m1[3];
+        for (int ax = 0; ax < 3; ++ax) {
+            const bool diff = (cls >> ax) & 1;
+            const double h = d->dx[ax];
+            k1[ax] = (diff ? -1.0 : 1.0) / h;
+            m1[ax] = diff ? h / 6.0 : h / 3.0;
+        }
+        T[cls] = three ? k1[0] * m1[1] * m1[2] + m1[0] * k1[1] * m1[2] + m1[0] * m1[1] * k1[2]
+                       : k1[0] * m1[1] + m1[0] * k1[1];
+    }
+}
 
 // Window geometry of k_f32_cg for a domain: one window per stencil plane (dz) covering the
 // rows [i0 - NN0 - 1, i0 + kTile + NN0 + 1) when that is shorter than three windows of
@@ -1647,51 +1626,21 @@ CgArgs cg_args(const Domain* d)
         ca.bpos[b] = w * ca.wlen + (int)(d->band_off[b] - ca.woff[w]);
     }
     ca.n = d->n;
-    // element-coefficient operator: khat windows hold the elements around the tile's rows,
-    // corner j = a + 2b + 4c at node offset a + NN0 b + NN0 NN1 c (all >= 0): one window per
-    // element plane (c) when NN0 is short, else one per (b, c); starts rounded down to 4 floats
+    // corner element j = a + 2b + 4c of a node at node offset a + NN0 b + NN0 NN1 c (all >= 0)
     const int nk = three ? 8 : 4;
-    const bool kmerged = nn0 + kTile + 1 <= 2 * (kTile + 1);
-    int64_t knom[4];
-    int64_t klen;
-    if (kmerged) {
-        ca.nkw = three ? 2 : 1;
-        klen = kTile + nn0 + 1;
-        for (int c = 0; c < ca.nkw; ++c) knom[c] = c * nn01;
-    } else {
-        ca.nkw = three ? 4 : 2;
-        klen = kTile + 1;
-        for (int w = 0; w < ca.nkw; ++w) knom[w] = (w & 1) * nn0 + (w >> 1) * nn01;
-    }
-    ca.kwlen = (int)((klen + 3 + 3) & ~(int64_t)3);
-    for (int w = 0; w < ca.nkw; ++w) ca.kwoff[w] = (int)(knom[w] - (knom[w] & 3));
     for (int j = 0; j < 8; ++j) {
         const int a = j & 1, b = (j >> 1) & 1, c = j >> 2;
-        const int64_t delta = j < nk ? a + nn0 * b + nn01 * c : 0;
-        ca.kdelta[j] = (int)delta;
-        const int w = j < nk ? (kmerged ? c : b + 2 * c) : 0;
-        ca.kpos[j] = w * ca.kwlen + (int)(delta - ca.kwoff[w]);
+        ca.kdelta[j] = j < nk ? (int)(a + nn0 * b + nn01 * c) : 0;
     }
-    // Q1 stiffness of the reference box (exact 1D integrals; the 2-point Gauss rule of the
-    // assembly is exact for them): per axis K = 1/h (same node) or -1/h, M = h/3 or h/6
-    for (int cls = 0; cls < 8; ++cls) {
-        double k1[3], m1[3];
-        for (int ax = 0; ax < 3; ++ax) {
-            const bool diff = (cls >> ax) & 1;
-            const double h = d->dx[ax];
-            k1[ax] = (diff ? -1.0 : 1.0) / h;
-            m1[ax] = diff ? h / 6.0 : h / 3.0;
-        }
-        const double t = three ? k1[0] * m1[1] * m1[2] + m1[0] * k1[1] * m1[2] + m1[0] * m1[1] * k1[2]
-                               : k1[0] * m1[1] + m1[0] * k1[1];
-        ca.T[cls] = (float)t;
-    }
+    double T[8];
+    q1_table(d, T);
+    for (int cls = 0; cls < 8; ++cls) ca.T[cls] = (float)T[cls];
     return ca;
 }
 
-size_t cg_smem(const Domain* d, const CgArgs& ca, int stages, bool coef)
+size_t cg_smem(const Domain* d, const CgArgs& ca, int stages)
 {
-    const size_t mat = coef ? (size_t)ca.nkw * ca.kwlen : (size_t)d->nbands * kTile;
+    const size_t mat = (size_t)d->nbands * kTile;
     return sizeof(float) * (size_t)stages * (mat + 4 * (size_t)ca.nwin * ca.wlen);
 }
 
@@ -1708,14 +1657,13 @@ int max_dyn_smem(const void* kernel, int* out)
     return RG_OK;
 }
 
-template <int NB, int S, int CPS, bool COEF>
+template <int NB, int S, int CPS>
 int cg_attribute()
 {
     int lim = 0;
-    int rc = max_dyn_smem((const void*)k_f32_cg<NB, S, CPS, COEF>, &lim);
+    int rc = max_dyn_smem((const void*)k_f32_cg<NB, S, CPS>, &lim);
     if (rc) return rc;
-    RG_CHECK_CUDA(
-        cudaFuncSetAttribute(k_f32_cg<NB, S, CPS, COEF>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+    RG_CHECK_CUDA(cudaFuncSetAttribute(k_f32_cg<NB, S, CPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     return RG_OK;
 }
 
@@ -1724,10 +1672,8 @@ int tma_attributes()
     static bool done = false;
     if (!done) {
         int rc;
-        if ((rc = cg_attribute<27, 3, 1, false>()) || (rc = cg_attribute<27, 2, 2, false>()) ||
-            (rc = cg_attribute<9, 3, 1, false>()) || (rc = cg_attribute<9, 2, 2, false>()) ||
-            (rc = cg_attribute<27, 3, 2, true>()) || (rc = cg_attribute<27, 2, 2, true>()) ||
-            (rc = cg_attribute<9, 3, 2, true>()) || (rc = cg_attribute<9, 2, 2, true>()))
+        if ((rc = cg_attribute<27, 3, 1>()) || (rc = cg_attribute<27, 2, 2>()) || (rc = cg_attribute<9, 3, 1>()) ||
+            (rc = cg_attribute<9, 2, 2>()))
             return rc;
         RG_CHECK_CUDA(cudaFuncSetAttribute(k_band64_bulk<27, band64_stages<27>(), false>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1746,73 +1692,139 @@ int tma_attributes()
     return RG_OK;
 }
 
-template <int NB, int S, int CPS, bool COEF>
-const void* cg_kernel() { return (const void*)k_f32_cg<NB, S, CPS, COEF>; }
-
-const void* cg_kernel_for(int nb, int cfg, bool coef)
+const void* cg_kernel_for(int nb, int cfg)
 {
-    if (coef) {
-        if (nb == 27) return cfg == 0 ? cg_kernel<27, 3, 2, true>() : cg_kernel<27, 2, 2, true>();
-        return cfg == 0 ? cg_kernel<9, 3, 2, true>() : cg_kernel<9, 2, 2, true>();
-    }
-    if (nb == 27) return cfg == 0 ? cg_kernel<27, 3, 1, false>() : cg_kernel<27, 2, 2, false>();
-    return cfg == 0 ? cg_kernel<9, 3, 1, false>() : cg_kernel<9, 2, 2, false>();
+    if (nb == 27) return cfg == 0 ? (const void*)k_f32_cg<27, 3, 1> : (const void*)k_f32_cg<27, 2, 2>;
+    return cfg == 0 ? (const void*)k_f32_cg<9, 3, 1> : (const void*)k_f32_cg<9, 2, 2>;
 }
 
-// (stages, CTAs per SM) of configuration cfg of an operator
-const int* cg_cfg(int cfg, bool coef) { return coef ? kCoefCfg[cfg] : kSpmvCfg[cfg]; }
+// whether the state windows are one per stencil plane (x-lines shorter than about a tile)
+bool windows_merged(const Domain* d) { return 2 * d->nn[0] + kTile + 2 <= 3 * (kTile + 2); }
 
-// whether configuration cfg reaches its CTAs per SM with this domain's windows
+// whether configuration cfg may run on this domain: on the band copy, whether it reaches its CTAs
+// per SM with this domain's windows.  On the element coefficients every grid takes configuration
+// 1; 0 is refused on 3D grids with long x-lines, which rg_solver_set_config always refused there
 bool cg_config_fits(const Domain* d, int cfg, bool coef)
 {
-    const void* kern = cg_kernel_for(d->nbands, cfg, coef);
-    const size_t smem = cg_smem(d, cg_args(d), cg_cfg(cfg, coef)[0], coef);
+    if (coef) return cfg == 1 || d->dim == 2 || windows_merged(d);
+    const void* kern = cg_kernel_for(d->nbands, cfg);
+    const size_t smem = cg_smem(d, cg_args(d), kSpmvCfg[cfg][0]);
     int lim = 0;
     if (max_dyn_smem(kern, &lim) != RG_OK || smem > (size_t)lim) return false;
     int blocks = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, kTile + 32, smem) != cudaSuccess) return false;
-    return blocks >= cg_cfg(cfg, coef)[1];
+    return blocks >= kSpmvCfg[cfg][1];
 }
 
-// one launch of the fused FP32 iteration (mode 0) or of a segment start (mode 1, 2) with the
-// workspace's current operator (band copy, or element coefficients when w->coef_op)
-template <int NB, int S, int CPS, bool COEF>
+// one launch of the fused FP32 iteration on the band copy (mode 0) or of a segment start (mode 1, 2)
+template <int NB, int S, int CPS>
 void launch_cg_k(Matrix* m, const CgArgs& ca, int grid, size_t smem, int mode)
 {
     Workspace* w = m->ws;
-    const float* op = COEF ? m->coef.khat : m->band32;
-    RG_TIMED(T_F32_SPMV, (k_f32_cg<NB, S, CPS, COEF><<<grid, kTile + 32, smem, stream()>>>(
-                             op, ca, w->v4[0], w->v4[1], w->v4[0], w->v4[1], w->d32, rbuf(w), w->s, mode)));
+    RG_TIMED(T_F32_SPMV, (k_f32_cg<NB, S, CPS><<<grid, kTile + 32, smem, stream()>>>(
+                             m->band32, ca, w->v4[0], w->v4[1], w->v4[0], w->v4[1], w->d32, rbuf(w), w->s, mode)));
 }
 
 template <int NB>
 int launch_cg(Matrix* m, int cfg, int mode)
 {
     const Domain* d = m->dom;
-    const bool coef = m->ws->coef_op;
     const CgArgs ca = cg_args(d);
-    const int* sc = cg_cfg(cfg, coef);
     const int64_t ntiles = (d->n + kTile - 1) / kTile;
-    const int grid = (int)std::min<int64_t>(ntiles, (int64_t)sm_count() * sc[1]);
-    const size_t smem = cg_smem(d, ca, sc[0], coef);
-    if (coef) {
-        if (cfg == 0)
-            launch_cg_k<NB, 3, 2, true>(m, ca, grid, smem, mode);
-        else
-            launch_cg_k<NB, 2, 2, true>(m, ca, grid, smem, mode);
-    } else {
-        if (cfg == 0)
-            launch_cg_k<NB, 3, 1, false>(m, ca, grid, smem, mode);
-        else
-            launch_cg_k<NB, 2, 2, false>(m, ca, grid, smem, mode);
-    }
+    const int grid = (int)std::min<int64_t>(ntiles, (int64_t)sm_count() * kSpmvCfg[cfg][1]);
+    const size_t smem = cg_smem(d, ca, kSpmvCfg[cfg][0]);
+    if (cfg == 0)
+        launch_cg_k<NB, 3, 1>(m, ca, grid, smem, mode);
+    else
+        launch_cg_k<NB, 2, 2>(m, ca, grid, smem, mode);
     RG_CHECK_LAUNCH();
     return RG_OK;
 }
 
-int launch_spmv_cfg(Matrix* m, int cfg, int mode = 0)
+int launch_band_cfg(Matrix* m, int cfg, int mode = 0)
 {
     return m->dom->nbands == 27 ? launch_cg<27>(m, cfg, mode) : launch_cg<9>(m, cfg, mode);
+}
+
+// ---- the FP32 iteration on the element coefficients (rg_cg_coef.cuh)
+CoefCgArgs coef_cg_args(Matrix* m, int cfg)
+{
+    const Domain* d = m->dom;
+    Workspace* w = m->ws;
+    CoefCgArgs a{};
+    double T[8];
+    q1_table(d, T);
+    a.t = march_table<float>(d->dim, T);
+    a.g = march_geom(d->dim, d->nn, d->dim == 3 ? kCoefLines[cfg] : 1, std::min(sm_count(), kMailCtas),
+                     kCoefWarps[cfg]);
+    a.khat = m->coef.khat;
+    a.v[0] = w->v4[0];
+    a.v[1] = w->v4[1];
+    a.d = w->d32;
+    a.mail = w->mail;
+    return a;
+}
+
+template <int DIM, int NR, int W>
+int launch_coef_t(CoefCgArgs& a, Scal* s, unsigned long long* mail)
+{
+    RG_CHECK_CUDA(cudaMemsetAsync(mail, 0, kMailBytes, stream()));
+    void* args[] = {&a, &s};
+    cudaError_t e;
+    const int grid = march_ctas(a.g, std::min(sm_count(), kMailCtas));
+    RG_TIMED(T_F32_SPMV, (e = cudaLaunchCooperativeKernel((const void*)k_f32_cg_coef<DIM, NR, W>, dim3(grid),
+                                                          dim3(W * 32), args, 0, stream())));
+    RG_CHECK_CUDA(e);
+    return RG_OK;
+}
+
+// one launch of up to `iters` FP32 iterations on the element coefficients
+int launch_coef(Matrix* m, int cfg, int iters)
+{
+    Workspace* w = m->ws;
+    CoefCgArgs a = coef_cg_args(m, cfg);
+    a.max_iters = iters;
+    if (m->dom->dim == 3)
+        return cfg == 0 ? launch_coef_t<3, kCoefLines[0], kCoefWarps[0]>(a, w->s, w->mail)
+                        : launch_coef_t<3, kCoefLines[1], kCoefWarps[1]>(a, w->s, w->mail);
+    return cfg == 0 ? launch_coef_t<2, 1, kCoefWarps[0]>(a, w->s, w->mail)
+                    : launch_coef_t<2, 1, kCoefWarps[1]>(a, w->s, w->mail);
+}
+
+int launch_coef_start(Matrix* m, int mode)
+{
+    Workspace* w = m->ws;
+    const CoefCgArgs a = coef_cg_args(m, 1);
+    const int grid = grid_for((int64_t)a.g.strips * a.g.slabs * 32, 128, 8);
+    if (m->dom->dim == 3)
+        RG_TIMED(T_F32_SPMV, (k_f32_cg_coef_start<3><<<grid, 128, 0, stream()>>>(a, rbuf(w), w->s, mode)));
+    else
+        RG_TIMED(T_F32_SPMV, (k_f32_cg_coef_start<2><<<grid, 128, 0, stream()>>>(a, rbuf(w), w->s, mode)));
+    RG_CHECK_LAUNCH();
+    return RG_OK;
+}
+
+// FP32 iterations on the element coefficients until the device flags done
+int run_coef(Matrix* m, int cfg, long long cap, long long* iters, int* status)
+{
+    Workspace* w = m->ws;
+    // about 20 ms of iterations per launch
+    const double iter_s = (double)m->dom->n * 60 / 5.0e12 + 3e-6;
+    const int chunk = (int)std::min(std::max(0.02 / iter_s, 16.0), 8192.0);
+    long long launched = 0;
+    for (;;) {
+        int rc = launch_coef(m, cfg, chunk);
+        if (rc || (rc = read_scal(w))) return rc;
+        launched += chunk;
+        if (w->hs->done) break;
+        if (launched > cap + 2LL * chunk + 8) {
+            set_error("PCG iteration loop did not terminate");
+            return RG_TIMEOUT;
+        }
+    }
+    *iters = w->hs->iter;
+    *status = w->hs->status;
+    return RG_OK;
 }
 
 // the tuned configuration of the workspace's current operator
@@ -1872,9 +1884,15 @@ int tune_spmv(Matrix* m)
         w->hs->pk = 0;
         w->hs->norm = 1.0;
         if ((rc = write_scal_fields(w, 0.0, 1LL << 40, 0))) break;  // done = 0, no iteration cap
-        for (int k = 0; k < 2 && rc == RG_OK; ++k) rc = launch_spmv_cfg(m, cfg);
+        auto iterate = [&](int count) {
+            if (coef) return launch_coef(m, cfg, count);
+            int r = RG_OK;
+            for (int k = 0; k < count && r == RG_OK; ++k) r = launch_band_cfg(m, cfg);
+            return r;
+        };
+        rc = iterate(2);
         RG_CHECK_CUDA(cudaEventRecord(e0, stream()));
-        for (int k = 0; k < 8 && rc == RG_OK; ++k) rc = launch_spmv_cfg(m, cfg);
+        if (rc == RG_OK) rc = iterate(8);
         RG_CHECK_CUDA(cudaEventRecord(e1, stream()));
         RG_CHECK_CUDA(cudaEventSynchronize(e1));
         float ms = 0;
@@ -1897,7 +1915,7 @@ int f32_step(Matrix* m)
 {
     Workspace* w = m->ws;
     const int cfg = cfg_slot(w);
-    return launch_spmv_cfg(m, cfg < 0 ? 0 : cfg, 0);
+    return launch_band_cfg(m, cfg < 0 ? 0 : cfg, 0);
 }
 
 // balance (first solve only) and the preconditioner data (paso Solver.cpp:98,177)
@@ -2057,7 +2075,7 @@ int solve_f32(Matrix* m, const rg_solver_opts* o, OuterState& st, rg_diag& dg)
     Workspace* w = m->ws;
     const int64_t n = m->dom->n;
     const int eg = grid_for(n, kThreads, 8);
-    const int chunk = chunk_for(n, w->coef_op ? 4 + 40 : 4 * 27 + 40);  // bytes per row of an iteration
+    const int chunk = chunk_for(n, 4 * 27 + 40);  // bytes per row of a band iteration
     // segment reduction factor: 1e-2 keeps the FP32 recurrence within a few ulps of the
     // true residual (smaller factors let it drift and cost iterations)
     const double seg = std::fmin(std::fmax(o->inner_tolerance > 0 ? o->inner_tolerance : 1e-2, 1e-4), 0.5);
@@ -2090,7 +2108,8 @@ int solve_f32(Matrix* m, const rg_solver_opts* o, OuterState& st, rg_diag& dg)
         w->hs->status = ST_RUN;
         RG_CHECK_CUDA(cudaMemcpyAsync(&w->s->status, &w->hs->status, sizeof(int), cudaMemcpyHostToDevice, stream()));
         const int cfg = cfg_slot(w);
-        if ((rc = launch_spmv_cfg(m, cfg < 0 ? 0 : cfg, first ? 1 : 2))) return rc;
+        rc = w->coef_op ? launch_coef_start(m, first ? 1 : 2) : launch_band_cfg(m, cfg < 0 ? 0 : cfg, first ? 1 : 2);
+        if (rc) return rc;
         if ((rc = read_scal(w))) return rc;
         if (w->hs->status == ST_BREAK || w->hs->status == ST_TIMEOUT) {
             bool restart = false;
@@ -2105,7 +2124,9 @@ int solve_f32(Matrix* m, const rg_solver_opts* o, OuterState& st, rg_diag& dg)
         if ((rc = write_scal_fields(w, tol, cap > 0 ? cap : 1, 0))) return rc;
         long long it = 0;
         int dst = ST_RUN;
-        if ((rc = run_until_done(m, 2, f32_step, chunk, cap, &it, &dst))) return rc;
+        rc = w->coef_op ? run_coef(m, cfg < 0 ? 1 : cfg, cap, &it, &dst)
+                        : run_until_done(m, 2, f32_step, chunk, cap, &it, &dst);
+        if (rc) return rc;
         st.totIter += it;
         done_iters += it;
         if (dst == ST_TIMEOUT) {
@@ -2114,8 +2135,8 @@ int solve_f32(Matrix* m, const rg_solver_opts* o, OuterState& st, rg_diag& dg)
         }
         // fold the FP32 correction into x and test the FP64 true residual
         if (w->coef_op)
-            RG_TIMED(T_VECTOR, (k_fold_correction_unbalance<<<eg, kThreads, 0, stream()>>>(n, w->x, w->d32, m->bv,
-                                                                                          scale)));
+            RG_TIMED(T_VECTOR, (k_fold_correction_unbalance<<<eg, kThreads, 0, stream()>>>(
+                                   n, w->x, w->d32, w->v4[0], w->v4[1], m->bv, w->s, scale)));
         else
             RG_TIMED(T_VECTOR, (k_fold_correction<<<eg, kThreads, 0, stream()>>>(n, w->x, w->d32, scale)));
         RG_CHECK_LAUNCH();
@@ -2330,7 +2351,6 @@ int solve_impl(Matrix* m, const double* rhs, double* x, const rg_solver_opts* o,
     bool coef = false;
     if (fp32 && o->layout == RG_LAYOUT_COEF && (rc = coef_usable(m, &coef))) return rc;
     if ((rc = prepare(m, fp32 && !coef, band64))) return rc;
-    if (coef && (rc = tma_attributes())) return rc;
     w->band64 = band64;
     w->coef_op = coef;
     dg.inner_operator = coef ? 1 : 0;
