@@ -9,8 +9,12 @@
 // ripley/src/DefaultAssembler3D.cpp:152-2226).  Rows of a CTA are contiguous in the
 // CSR arrays, so each CTA stages its rows in shared memory and writes them back with
 // coalesced stores.
+#include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstring>
+#include <mutex>
+#include <type_traits>
 
 #include "rg_internal.cuh"
 
@@ -145,6 +149,7 @@ __global__ void __launch_bounds__(kRowsPerCta) k_pattern(const __grid_constant__
 struct CoefArg {
     const double* p;
     int kind;
+    int wide;  // the array starts on a 16-byte boundary
 };
 
 // Element-matrix tables integrated over the Gauss points, for operator coefficients that
@@ -168,135 +173,202 @@ struct AsmArgs {
     const int32_t* ptr;
     double* val;
     double* rhs;
+    int place[6], stride;  // a staged element's doubles: where each coefficient starts, and from one to the next
 };
 
-// coefficient data point of element e at Gauss point q (SIZE values)
-template <int SIZE, int NQ>
-__device__ __forceinline__ const double* coef_ptr(const CoefArg& c, int64_t e, int q)
+// How a warp assembles.  Lane l works on row base + l - 1 (31 rows: lane 0 only helps) and, per line of
+// elements (sy, sz) beside the rows, on the element right of its row: that element is the left one of
+// the next lane's row, so a lane forms its element matrix's rows for both nodes from one reading of the
+// coefficients and hands the second on by shuffles.  Across the ends of x-lines and planes the elements
+// of a warp's valid lanes still follow one another in memory; their data points are copied with
+// cp.async into the warp's own buffer, in 16-byte pieces, one run per element and coefficient, padded so
+// that lanes reading 16 bytes of consecutive elements meet no bank conflict.  Half of the Gauss points
+// are copied at a time: 8 warps per SM stay resident, which the 234 registers allow as well.  (Two
+// points at a time into one of two buffers, ahead of the arithmetic, was slower: 1.23 ms; the copies'
+// instructions count more than their latency.)
+//
+// Read directly instead, every load of a lane lies 72 to 576 bytes from its neighbour's (up to 32
+// wavefronts a load), and each of an element's 8 nodes reads it again: 3.08 ms at 96^3 with all six
+// coefficients at the Gauss points, 0.99 ms now (1.4 GB of HBM traffic, 0.21 ms; 0.20 ms of FP64 pipe).
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+
+template <int BYTES>
+__device__ __forceinline__ void copy_async(uint32_t dst, const void* src)
 {
-    if (c.kind == RG_COEF_EXPANDED) return c.p + ((size_t)e * NQ + q) * SIZE;
-    if (c.kind == RG_COEF_PER_ELEMENT) return c.p + (size_t)e * SIZE;
-    return c.p;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
 }
 
-// Row R of the element matrix and vector of element e:
-//   em[c] = sum_q W (A_ij G_Ri G_cj + B_i G_Ri N_c + C_j N_R G_cj + D N_R N_c)
-//   f     = sum_q W (X_i G_Ri + Y N_R)
-// UNI: A, B, C, D are constant over the element, em comes from the integrated tables.
-template <int DIM, int NQ, int R, bool UNI>
-__device__ __forceinline__ void element_row(const AsmArgs& a, int64_t e, double (&em)[1 << DIM],
-                                            double& f)
+constexpr int kAsmRows = 31, kAsmWarps = 4;  // rows per warp, warps per CTA
+
+// Gauss points per stage: half of them, or the one of the 1-point rule
+template <int NQ>
+constexpr int asm_points() { return NQ >= 4 ? NQ / 2 : 1; }
+
+// doubles per element and stage of coefficient j
+template <int DIM, int NQ, int J>
+constexpr int asm_run()
 {
-    if constexpr (UNI) {
-        constexpr int NK = 1 << DIM;
-        const CoefArg& A = a.c[0];
-        const CoefArg& B = a.c[1];
-        const CoefArg& C = a.c[2];
-        const CoefArg& D = a.c[3];
-        const CoefArg& X = a.c[4];
-        const CoefArg& Y = a.c[5];
-#pragma unroll
-        for (int c = 0; c < NK; ++c) em[c] = 0.0;
-        if (A.kind) {
-            const double* ap = coef_ptr<DIM * DIM, 1>(A, e, 0);
-#pragma unroll
-            for (int j = 0; j < DIM; ++j)
-#pragma unroll
-                for (int i = 0; i < DIM; ++i) {
-                    const double aij = __ldg(ap + i + DIM * j);
-#pragma unroll
-                    for (int c = 0; c < NK; ++c) em[c] = fma(aij, a.u.SA[i][j][R][c], em[c]);
+    return (J == 0 ? DIM * DIM : (J == 3 || J == 5 ? 1 : DIM)) * asm_points<NQ>();
+}
+
+// copies `count` elements' part of half h of one coefficient: element e's run to dst + e * stride doubles.
+// A CONSTANT or PER_ELEMENT coefficient is laid out as if given at each point.
+template <int DIM, int NQ, int J>
+__device__ __forceinline__ void stage_coef(const CoefArg& c, int64_t e0, int count, int h, uint32_t dst, int stride,
+                                           int lane)
+{
+    constexpr int size = J == 0 ? DIM * DIM : (J == 3 || J == 5 ? 1 : DIM);
+    constexpr int N = asm_run<DIM, NQ, J>();
+    if (!c.kind) return;
+    if (c.kind == RG_COEF_EXPANDED) {
+        constexpr int all = size * NQ;
+        const double* src = c.p + e0 * all + h * N;
+        if constexpr (N % 2 == 0 && all % 2 == 0) {
+            if (c.wide) {
+                for (int k = lane; k < count * (N / 2); k += 32) {
+                    const int e = k / (N / 2), i = k - e * (N / 2);
+                    copy_async<16>(dst + (uint32_t)(e * stride + 2 * i) * 8u, src + e * all + 2 * i);
                 }
-        }
-        if (B.kind) {
-            const double* bp = coef_ptr<DIM, 1>(B, e, 0);
-#pragma unroll
-            for (int i = 0; i < DIM; ++i) {
-                const double bi = __ldg(bp + i);
-#pragma unroll
-                for (int c = 0; c < NK; ++c) em[c] = fma(bi, a.u.SB[i][R][c], em[c]);
+                return;
             }
         }
-        if (C.kind) {
-            const double* cp = coef_ptr<DIM, 1>(C, e, 0);
-#pragma unroll
-            for (int j = 0; j < DIM; ++j) {
-                const double cj = __ldg(cp + j);
-#pragma unroll
-                for (int c = 0; c < NK; ++c) em[c] = fma(cj, a.u.SC[j][R][c], em[c]);
-            }
+        for (int k = lane; k < count * N; k += 32) {
+            const int e = k / N, i = k - e * N;
+            copy_async<8>(dst + (uint32_t)(e * stride + i) * 8u, src + e * all + i);
         }
-        if (D.kind) {
-            const double dd = __ldg(coef_ptr<1, 1>(D, e, 0));
-#pragma unroll
-            for (int c = 0; c < NK; ++c) em[c] = fma(dd, a.u.M[R][c], em[c]);
+    } else {
+        const double* src = c.kind == RG_COEF_PER_ELEMENT ? c.p + e0 * size : c.p;
+        const int step = c.kind == RG_COEF_PER_ELEMENT ? size : 0;
+        for (int k = lane; k < count * N; k += 32) {
+            const int e = k / N, i = k - e * N;
+            copy_async<8>(dst + (uint32_t)(e * stride + i) * 8u, src + e * step + i % size);
         }
-        f = 0.0;
-        if (X.kind || Y.kind) {
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-                double fq = 0.0;
-                if (Y.kind) fq = __ldg(coef_ptr<1, NQ>(Y, e, q)) * a.t.N[q][R];
-                if (X.kind) {
-                    const double* xp = coef_ptr<DIM, NQ>(X, e, q);
-#pragma unroll
-                    for (int i = 0; i < DIM; ++i) fq = fma(__ldg(xp + i), a.t.G[q][R][i], fq);
-                }
-                f = fma(a.t.W, fq, f);
-            }
-        }
-        return;
     }
-    constexpr int NK = 1 << DIM, D2 = DIM * DIM;
-    const CoefArg& A = a.c[0];
-    const CoefArg& B = a.c[1];
-    const CoefArg& C = a.c[2];
-    const CoefArg& D = a.c[3];
-    const CoefArg& X = a.c[4];
-    const CoefArg& Y = a.c[5];
+}
+
+// N doubles of an element's run, in 16-byte reads (p is on a 16-byte boundary)
+template <int N>
+__device__ __forceinline__ void read_run(const double* p, double (&v)[N])
+{
 #pragma unroll
-    for (int c = 0; c < NK; ++c) em[c] = 0.0;
-    f = 0.0;
+    for (int k = 0; k + 1 < N; k += 2) {
+        const double2 t = reinterpret_cast<const double2*>(p)[k / 2];
+        v[k] = t.x;
+        v[k + 1] = t.y;
+    }
+    if (N & 1) v[N - 1] = p[N - 1];
+}
+
+// local number of a row's node in the element right of it on line `line` = sy + 2 sz
+template <int DIM>
+__host__ __device__ constexpr int line_node(int line)
+{
+    return 2 * (1 - (line & 1)) + (DIM == 3 ? 4 * (1 - (line >> 1)) : 0);
+}
+
+// a shape function and its gradient at a Gauss point
+struct Shape {
+    double n, g[3];
+};
+__device__ __forceinline__ Shape shape_at(const double* tab, int q, int k)
+{
+    const double2* t = reinterpret_cast<const double2*>(tab + (q * 8 + k) * 4);
+    const double2 a = t[0], b = t[1];
+    return Shape{a.x, {a.y, b.x, b.y}};
+}
+
+// The rows of local nodes r0 and r0 + 1 of a staged element (its data at el), half h of the points:
+//   em[r][c] += sum_q W (A_ij G_Ri G_cj + B_i G_Ri N_c + C_j N_R G_cj + D N_R N_c)
+//   f[r]     += sum_q W (X_i G_Ri + Y N_R)
+template <int DIM, int NQ>
+__device__ __forceinline__ void element_rows(const AsmArgs& a, const double* tab, const double* el, int h, int r0,
+                                             double (&em)[2][1 << DIM], double (&f)[2])
+{
+    constexpr int NK = 1 << DIM, D2 = DIM * DIM, NP = asm_points<NQ>(), G = NP >= 2 ? 2 : 1;
+#pragma unroll 1
+    for (int p0 = 0; p0 < NP; p0 += G) {
+        double s[G][2][DIM], t0[G][2];
+        Shape R[G][2];
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-        const double NR = a.t.N[q][R];
-        double s[DIM];
+        for (int g = 0; g < G; ++g)
 #pragma unroll
-        for (int j = 0; j < DIM; ++j) s[j] = 0.0;
-        double t0 = 0.0;
-        if (A.kind) {
-            const double* ap = coef_ptr<D2, NQ>(A, e, q);
+            for (int r = 0; r < 2; ++r) {
+                R[g][r] = shape_at(tab, h * NP + p0 + g, r0 + r);
+                t0[g][r] = 0.0;
 #pragma unroll
-            for (int j = 0; j < DIM; ++j)
+                for (int j = 0; j < DIM; ++j) s[g][r][j] = 0.0;
+            }
+        if (a.c[0].kind) {
+            double v[G * D2];
+            read_run<G * D2>(el + a.place[0] + p0 * D2, v);
 #pragma unroll
-                for (int i = 0; i < DIM; ++i) s[j] = fma(__ldg(ap + i + DIM * j), a.t.G[q][R][i], s[j]);
+            for (int g = 0; g < G; ++g)
+#pragma unroll
+                for (int r = 0; r < 2; ++r)
+#pragma unroll
+                    for (int j = 0; j < DIM; ++j)
+#pragma unroll
+                        for (int i = 0; i < DIM; ++i) s[g][r][j] = fma(v[g * D2 + i + DIM * j], R[g][r].g[i], s[g][r][j]);
         }
-        if (C.kind) {
-            const double* cp = coef_ptr<DIM, NQ>(C, e, q);
+        if (a.c[2].kind) {
+            double v[G * DIM];
+            read_run<G * DIM>(el + a.place[2] + p0 * DIM, v);
 #pragma unroll
-            for (int j = 0; j < DIM; ++j) s[j] = fma(__ldg(cp + j), NR, s[j]);
+            for (int g = 0; g < G; ++g)
+#pragma unroll
+                for (int r = 0; r < 2; ++r)
+#pragma unroll
+                    for (int j = 0; j < DIM; ++j) s[g][r][j] = fma(v[g * DIM + j], R[g][r].n, s[g][r][j]);
         }
-        if (B.kind) {
-            const double* bp = coef_ptr<DIM, NQ>(B, e, q);
+        if (a.c[1].kind) {
+            double v[G * DIM];
+            read_run<G * DIM>(el + a.place[1] + p0 * DIM, v);
 #pragma unroll
-            for (int i = 0; i < DIM; ++i) t0 = fma(__ldg(bp + i), a.t.G[q][R][i], t0);
+            for (int g = 0; g < G; ++g)
+#pragma unroll
+                for (int r = 0; r < 2; ++r)
+#pragma unroll
+                    for (int i = 0; i < DIM; ++i) t0[g][r] = fma(v[g * DIM + i], R[g][r].g[i], t0[g][r]);
         }
-        if (D.kind) t0 = fma(__ldg(coef_ptr<1, NQ>(D, e, q)), NR, t0);
+        if (a.c[3].kind) {
+            double v[G];
+            read_run<G>(el + a.place[3] + p0, v);
 #pragma unroll
-        for (int c = 0; c < NK; ++c) {
-            double v = t0 * a.t.N[q][c];
+            for (int g = 0; g < G; ++g)
 #pragma unroll
-            for (int j = 0; j < DIM; ++j) v = fma(s[j], a.t.G[q][c][j], v);
-            em[c] = fma(a.t.W, v, em[c]);
+                for (int r = 0; r < 2; ++r) t0[g][r] = fma(v[g], R[g][r].n, t0[g][r]);
         }
-        double fq = 0.0;
-        if (Y.kind) fq = __ldg(coef_ptr<1, NQ>(Y, e, q)) * NR;
-        if (X.kind) {
-            const double* xp = coef_ptr<DIM, NQ>(X, e, q);
+        if (a.c[4].kind || a.c[5].kind) {
+            double y[G], x[G * DIM];
 #pragma unroll
-            for (int i = 0; i < DIM; ++i) fq = fma(__ldg(xp + i), a.t.G[q][R][i], fq);
+            for (int g = 0; g < G; ++g) y[g] = 0.0;
+#pragma unroll
+            for (int k = 0; k < G * DIM; ++k) x[k] = 0.0;
+            if (a.c[5].kind) read_run<G>(el + a.place[5] + p0, y);
+            if (a.c[4].kind) read_run<G * DIM>(el + a.place[4] + p0 * DIM, x);
+#pragma unroll
+            for (int g = 0; g < G; ++g)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    double fq = y[g] * R[g][r].n;
+#pragma unroll
+                    for (int i = 0; i < DIM; ++i) fq = fma(x[g * DIM + i], R[g][r].g[i], fq);
+                    f[r] = fma(a.t.W, fq, f[r]);
+                }
         }
-        f = fma(a.t.W, fq, f);
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+#pragma unroll
+            for (int c = 0; c < NK; ++c) {
+                const Shape k = shape_at(tab, h * NP + p0 + g, c);
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    double v = t0[g][r] * k.n;
+#pragma unroll
+                    for (int j = 0; j < DIM; ++j) v = fma(s[g][r][j], k.g[j], v);
+                    em[r][c] = fma(a.t.W, v, em[r][c]);
+                }
+            }
     }
 }
 
@@ -309,57 +381,16 @@ __host__ __device__ constexpr int band_of(int sx, int sy, int sz, int c)
                     : (sx + (c & 1)) + 3 * (sy + ((c >> 1) & 1));
 }
 
-template <int DIM, int NQ, bool UNI, int SX, int SY, int SZ>
-__device__ __forceinline__ void add_element(const AsmArgs& a, int64_t x, int64_t y, int64_t z,
-                                            double (&acc)[DIM == 3 ? 27 : 9], double& facc)
-{
-    constexpr int NK = 1 << DIM;
-    const int64_t ex = x - 1 + SX, ey = y - 1 + SY, ez = z - 1 + SZ;
-    if (ex < 0 || ex >= a.NE0 || ey < 0 || ey >= a.NE1) return;
-    if (DIM == 3 && (ez < 0 || ez >= a.NE2)) return;
-    const int64_t e = ex + a.NE0 * ey + (DIM == 3 ? a.NE0 * a.NE1 * ez : 0);
-    constexpr int R = (1 - SX) + 2 * (1 - SY) + (DIM == 3 ? 4 * (1 - SZ) : 0);
-    double em[NK], f;
-    element_row<DIM, NQ, R, UNI>(a, e, em, f);
-#pragma unroll
-    for (int c = 0; c < NK; ++c) acc[band_of<DIM>(SX, SY, SZ, c)] += em[c];
-    facc += f;
-}
-
-// NQ = 2^DIM Gauss points (assemblePDESingle) or 1, the element centre
-// (assemblePDESingleReduced); the tables in `a.t` hold the matching rule
-template <int DIM, int NQ, bool UNI>
-__global__ void __launch_bounds__(kRowsPerCta) k_assemble(const __grid_constant__ AsmArgs a)
+// the CTA's rows [row0, row1), one per owning thread (row i at (x, y, z)), to the matrix through `stage`
+template <int DIM>
+__device__ __forceinline__ void write_rows(const AsmArgs& a, const double (&acc)[DIM == 3 ? 27 : 9], int64_t i, bool owned,
+                                           int64_t x, int64_t y, int64_t z, int64_t row0, int64_t row1, double* stage)
 {
     constexpr int NB = DIM == 3 ? 27 : 9;
-    __shared__ double stage[kRowsPerCta * NB];
-    const int64_t row0 = (int64_t)blockIdx.x * kRowsPerCta;
-    const int64_t row1 = min(row0 + kRowsPerCta, a.n);
-    const int64_t i = row0 + threadIdx.x;
-    double acc[NB];
-#pragma unroll
-    for (int b = 0; b < NB; ++b) acc[b] = 0.0;
-    double facc = 0.0;
-    int64_t x = 0, y = 0, z = 0;
-    if (i < a.n) {
-        x = i % a.NN0;
-        y = (i / a.NN0) % a.NN1;
-        z = DIM == 3 ? i / (a.NN0 * a.NN1) : 0;
-        add_element<DIM, NQ, UNI, 0, 0, 0>(a, x, y, z, acc, facc);
-        add_element<DIM, NQ, UNI, 1, 0, 0>(a, x, y, z, acc, facc);
-        add_element<DIM, NQ, UNI, 0, 1, 0>(a, x, y, z, acc, facc);
-        add_element<DIM, NQ, UNI, 1, 1, 0>(a, x, y, z, acc, facc);
-        if (DIM == 3) {
-            add_element<DIM, NQ, UNI, 0, 0, 1>(a, x, y, z, acc, facc);
-            add_element<DIM, NQ, UNI, 1, 0, 1>(a, x, y, z, acc, facc);
-            add_element<DIM, NQ, UNI, 0, 1, 1>(a, x, y, z, acc, facc);
-            add_element<DIM, NQ, UNI, 1, 1, 1>(a, x, y, z, acc, facc);
-        }
-        if (a.rhs) a.rhs[i] += facc;
-    }
     if (!a.val) return;  // uniform across the CTA
+    __syncthreads();     // the coefficient buffers become the rows' staging
     const int64_t base = a.ptr[row0];
-    if (i < a.n) {
+    if (owned) {
         int64_t k = a.ptr[i] - base;
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
@@ -371,7 +402,217 @@ __global__ void __launch_bounds__(kRowsPerCta) k_assemble(const __grid_constant_
     }
     __syncthreads();
     const int64_t end = a.ptr[row1];
-    for (int64_t t = threadIdx.x; t < end - base; t += kRowsPerCta) a.val[base + t] += stage[t];
+    // (a constant stride, so that the compiler unrolls: the loop is bound by the latency of its reads)
+    constexpr int kThreads = 128;
+    static_assert(kThreads == kRowsPerCta && kThreads == kAsmWarps * 32, "both kernels run blocks of 128");
+    for (int64_t t = threadIdx.x; t < end - base; t += kThreads) a.val[base + t] += stage[t];
+}
+
+// coefficient data point of element e at Gauss point q (SIZE values)
+template <int SIZE, int NQ>
+__device__ __forceinline__ const double* coef_ptr(const CoefArg& c, int64_t e, int q)
+{
+    if (c.kind == RG_COEF_EXPANDED) return c.p + ((size_t)e * NQ + q) * SIZE;
+    if (c.kind == RG_COEF_PER_ELEMENT) return c.p + (size_t)e * SIZE;
+    return c.p;
+}
+
+// NQ = 2^DIM Gauss points (assemblePDESingle) or 1, the element centre
+// (assemblePDESingleReduced); the tables in `a.t` hold the matching rule
+template <int DIM, int NQ>
+__global__ void __launch_bounds__(kAsmWarps * 32) k_assemble(const __grid_constant__ AsmArgs a)
+{
+    constexpr int NB = DIM == 3 ? 27 : 9, NK = 1 << DIM, kRows = kAsmRows * kAsmWarps;
+    // the shape functions, then the warps' coefficient buffers or the CTA's rows on their way out
+    extern __shared__ __align__(16) double smem_asm[];
+    double* tab = smem_asm;
+    double* stage = smem_asm + NQ * 8 * 4;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int k = threadIdx.x; k < NQ * 8 * 4; k += blockDim.x) {
+        const int q = k / 32, c = (k / 4) % 8, d = k % 4;
+        tab[k] = d == 0 ? a.t.N[q][c] : a.t.G[q][c][d - 1];
+    }
+    __syncthreads();
+    constexpr int kStages = NQ / asm_points<NQ>(), kLines = DIM == 3 ? 4 : 2;
+    double* buf = stage + (size_t)warp * 32 * a.stride;  // 32 elements
+    const uint32_t dst = smem_addr(buf);
+    const int64_t row0 = (int64_t)blockIdx.x * kRows, row1 = min(row0 + kRows, a.n);
+    const int64_t i = row0 + warp * kAsmRows + lane - 1;
+    const bool row = i >= 0 && i < a.n;
+    const int64_t x = row ? i % a.NN0 : 0, y = row ? (i / a.NN0) % a.NN1 : 0;
+    const int64_t z = DIM == 3 && row ? i / (a.NN0 * a.NN1) : 0;
+    double acc[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) acc[b] = 0.0;
+    double facc = 0.0;
+#pragma unroll 1
+    for (int line = 0; line < kLines; ++line) {
+        const int64_t ey = y - 1 + (line & 1), ez = DIM == 3 ? z - 1 + (line >> 1) : 0;
+        const int64_t e = x + a.NE0 * ey + a.NE0 * a.NE1 * ez;
+        const bool mine = row && x < a.NE0 && ey >= 0 && ey < a.NE1 && ez >= 0 && ez < a.NE2;
+        // the first element of the warp's (element counts fit 31 bits)
+        const unsigned first = __reduce_min_sync(0xffffffffu, mine ? (unsigned)e : 0xffffffffu);
+        if (first == 0xffffffffu) continue;
+        const int count = (int)min((int64_t)32, a.NE0 * a.NE1 * a.NE2 - (int64_t)first);
+        const double* el = buf + (mine ? (int)(e - first) : 0) * a.stride;
+        double em[2][NK], f[2] = {0.0, 0.0};
+#pragma unroll
+        for (int c = 0; c < NK; ++c) em[0][c] = em[1][c] = 0.0;
+#pragma unroll 1
+        for (int h = 0; h < kStages; ++h) {
+            __syncwarp();  // the stage before was read by all lanes
+            stage_coef<DIM, NQ, 0>(a.c[0], first, count, h, dst + a.place[0] * 8, a.stride, lane);
+            stage_coef<DIM, NQ, 1>(a.c[1], first, count, h, dst + a.place[1] * 8, a.stride, lane);
+            stage_coef<DIM, NQ, 2>(a.c[2], first, count, h, dst + a.place[2] * 8, a.stride, lane);
+            stage_coef<DIM, NQ, 3>(a.c[3], first, count, h, dst + a.place[3] * 8, a.stride, lane);
+            stage_coef<DIM, NQ, 4>(a.c[4], first, count, h, dst + a.place[4] * 8, a.stride, lane);
+            stage_coef<DIM, NQ, 5>(a.c[5], first, count, h, dst + a.place[5] * 8, a.stride, lane);
+            asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory");
+            __syncwarp();
+            if (mine) element_rows<DIM, NQ>(a, tab, el, h, line_node<DIM>(line), em, f);
+        }
+        // the row of the element's right node belongs to the next lane
+        double left[NK];
+#pragma unroll
+        for (int c = 0; c < NK; ++c) left[c] = __shfl_up_sync(0xffffffffu, em[1][c], 1);
+        const double fl = __shfl_up_sync(0xffffffffu, f[1], 1);
+        auto add = [&](auto l_) {
+            constexpr int SY = decltype(l_)::value & 1, SZ = decltype(l_)::value >> 1;
+#pragma unroll
+            for (int c = 0; c < NK; ++c) {
+                acc[band_of<DIM>(0, SY, SZ, c)] += left[c];
+                acc[band_of<DIM>(1, SY, SZ, c)] += em[0][c];
+            }
+        };
+        if (line == 0)
+            add(std::integral_constant<int, 0>());
+        else if (line == 1)
+            add(std::integral_constant<int, 1>());
+        else if (DIM == 3 && line == 2)
+            add(std::integral_constant<int, DIM == 3 ? 2 : 0>());
+        else
+            add(std::integral_constant<int, DIM == 3 ? 3 : 0>());
+        facc += fl + f[0];
+    }
+    const bool owned = row && lane >= 1;
+    if (owned && a.rhs) a.rhs[i] += facc;
+    write_rows<DIM>(a, acc, i, owned, x, y, z, row0, row1, stage);
+}
+
+// A, B, C, D constant over each element: em from the integrated tables
+template <int DIM, int NQ, int R>
+__device__ __forceinline__ void element_row_uni(const AsmArgs& a, int64_t e, double (&em)[1 << DIM], double& f)
+{
+    constexpr int NK = 1 << DIM;
+    const CoefArg& A = a.c[0];
+    const CoefArg& B = a.c[1];
+    const CoefArg& C = a.c[2];
+    const CoefArg& D = a.c[3];
+    const CoefArg& X = a.c[4];
+    const CoefArg& Y = a.c[5];
+#pragma unroll
+    for (int c = 0; c < NK; ++c) em[c] = 0.0;
+    if (A.kind) {
+        const double* ap = coef_ptr<DIM * DIM, 1>(A, e, 0);
+#pragma unroll
+        for (int j = 0; j < DIM; ++j)
+#pragma unroll
+            for (int i = 0; i < DIM; ++i) {
+                const double aij = __ldg(ap + i + DIM * j);
+#pragma unroll
+                for (int c = 0; c < NK; ++c) em[c] = fma(aij, a.u.SA[i][j][R][c], em[c]);
+            }
+    }
+    if (B.kind) {
+        const double* bp = coef_ptr<DIM, 1>(B, e, 0);
+#pragma unroll
+        for (int i = 0; i < DIM; ++i) {
+            const double bi = __ldg(bp + i);
+#pragma unroll
+            for (int c = 0; c < NK; ++c) em[c] = fma(bi, a.u.SB[i][R][c], em[c]);
+        }
+    }
+    if (C.kind) {
+        const double* cp = coef_ptr<DIM, 1>(C, e, 0);
+#pragma unroll
+        for (int j = 0; j < DIM; ++j) {
+            const double cj = __ldg(cp + j);
+#pragma unroll
+            for (int c = 0; c < NK; ++c) em[c] = fma(cj, a.u.SC[j][R][c], em[c]);
+        }
+    }
+    if (D.kind) {
+        const double dd = __ldg(coef_ptr<1, 1>(D, e, 0));
+#pragma unroll
+        for (int c = 0; c < NK; ++c) em[c] = fma(dd, a.u.M[R][c], em[c]);
+    }
+    f = 0.0;
+    if (X.kind || Y.kind) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            double fq = 0.0;
+            if (Y.kind) fq = __ldg(coef_ptr<1, NQ>(Y, e, q)) * a.t.N[q][R];
+            if (X.kind) {
+                const double* xp = coef_ptr<DIM, NQ>(X, e, q);
+#pragma unroll
+                for (int i = 0; i < DIM; ++i) fq = fma(__ldg(xp + i), a.t.G[q][R][i], fq);
+            }
+            f = fma(a.t.W, fq, f);
+        }
+    }
+}
+
+template <int DIM, int NQ, int SX, int SY, int SZ>
+__device__ __forceinline__ void add_element(const AsmArgs& a, int64_t x, int64_t y, int64_t z,
+                                            double (&acc)[DIM == 3 ? 27 : 9], double& facc)
+{
+    constexpr int NK = 1 << DIM;
+    const int64_t ex = x - 1 + SX, ey = y - 1 + SY, ez = z - 1 + SZ;
+    if (ex < 0 || ex >= a.NE0 || ey < 0 || ey >= a.NE1) return;
+    if (DIM == 3 && (ez < 0 || ez >= a.NE2)) return;
+    const int64_t e = ex + a.NE0 * ey + (DIM == 3 ? a.NE0 * a.NE1 * ez : 0);
+    constexpr int R = (1 - SX) + 2 * (1 - SY) + (DIM == 3 ? 4 * (1 - SZ) : 0);
+    double em[NK], f;
+    element_row_uni<DIM, NQ, R>(a, e, em, f);
+#pragma unroll
+    for (int c = 0; c < NK; ++c) acc[band_of<DIM>(SX, SY, SZ, c)] += em[c];
+    facc += f;
+}
+
+// One thread per row sums the rows of its adjacent elements; few values per element, read directly.
+// (Sharing an element between the lanes of its two nodes as k_assemble does takes twice the registers:
+// 0.95 against 0.69 ms at 128^3 with A and Y per element.)
+template <int DIM, int NQ>
+__global__ void __launch_bounds__(kRowsPerCta) k_assemble_uni(const __grid_constant__ AsmArgs a)
+{
+    constexpr int NB = DIM == 3 ? 27 : 9;
+    __shared__ double stage[kRowsPerCta * NB];
+    const int64_t row0 = (int64_t)blockIdx.x * kRowsPerCta;
+    const int64_t row1 = min(row0 + kRowsPerCta, a.n);
+    const int64_t i = row0 + threadIdx.x;
+    double acc[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) acc[b] = 0.0;
+    double facc = 0.0;
+    int64_t x = 0, y = 0, z = 0;
+    const bool owned = i < a.n;
+    if (owned) {
+        x = i % a.NN0;
+        y = (i / a.NN0) % a.NN1;
+        z = DIM == 3 ? i / (a.NN0 * a.NN1) : 0;
+        add_element<DIM, NQ, 0, 0, 0>(a, x, y, z, acc, facc);
+        add_element<DIM, NQ, 1, 0, 0>(a, x, y, z, acc, facc);
+        add_element<DIM, NQ, 0, 1, 0>(a, x, y, z, acc, facc);
+        add_element<DIM, NQ, 1, 1, 0>(a, x, y, z, acc, facc);
+        if (DIM == 3) {
+            add_element<DIM, NQ, 0, 0, 1>(a, x, y, z, acc, facc);
+            add_element<DIM, NQ, 1, 0, 1>(a, x, y, z, acc, facc);
+            add_element<DIM, NQ, 0, 1, 1>(a, x, y, z, acc, facc);
+            add_element<DIM, NQ, 1, 1, 1>(a, x, y, z, acc, facc);
+        }
+        if (a.rhs) a.rhs[i] += facc;
+    }
+    write_rows<DIM>(a, acc, i, owned, x, y, z, row0, row1, stage);
 }
 
 // ------------------------------------------------------------------ boundary assembly
@@ -540,6 +781,48 @@ int launch_pattern(Domain* d)
     return RG_OK;
 }
 
+namespace {
+
+template <int DIM, int NQ>
+int launch_assemble(AsmArgs& a)
+{
+    constexpr int run[6] = {asm_run<DIM, NQ, 0>(), asm_run<DIM, NQ, 1>(), asm_run<DIM, NQ, 2>(),
+                            asm_run<DIM, NQ, 3>(), asm_run<DIM, NQ, 4>(), asm_run<DIM, NQ, 5>()};
+    int total = 0;
+    for (int j = 0; j < 6; ++j) {
+        CoefArg& c = a.c[j];
+        a.place[j] = total;
+        if (c.kind) total += (run[j] + 1) & ~1;
+        c.wide = reinterpret_cast<uintptr_t>(c.p) % 16 == 0;
+    }
+    // 2 mod 4 doubles: the 16-byte reads of 8 consecutive elements cover all banks
+    a.stride = total % 4 == 2 ? total : total + 2;
+    constexpr int NB = DIM == 3 ? 27 : 9, kRows = kAsmRows * kAsmWarps;
+    const size_t smem =
+        sizeof(double) * (NQ * 8 * 4 + std::max((size_t)kRows * NB, (size_t)kAsmWarps * 32 * a.stride));
+    static std::once_flag once;
+    static cudaError_t attr = cudaSuccess;
+    std::call_once(once, [] {
+        attr = cudaFuncSetAttribute(k_assemble<DIM, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
+    });
+    RG_CHECK_CUDA(attr);
+    const int grid = (int)((a.n + kRows - 1) / kRows);
+    RG_TIMED(T_ASSEMBLE, (k_assemble<DIM, NQ><<<grid, kAsmWarps * 32, smem, stream()>>>(a)));
+    RG_CHECK_LAUNCH();
+    return RG_OK;
+}
+
+template <int DIM, int NQ>
+int launch_assemble_uni(const AsmArgs& a)
+{
+    const int grid = (int)((a.n + kRowsPerCta - 1) / kRowsPerCta);
+    RG_TIMED(T_ASSEMBLE, (k_assemble_uni<DIM, NQ><<<grid, kRowsPerCta, 0, stream()>>>(a)));
+    RG_CHECK_LAUNCH();
+    return RG_OK;
+}
+
+}  // namespace
+
 int assemble_single_impl(const Domain* d, double* val, double* rhs, const rg_coef* c[6], bool reduced)
 {
     AsmArgs a;
@@ -579,21 +862,9 @@ int assemble_single_impl(const Domain* d, double* val, double* rhs, const rg_coe
     a.val = addS ? val : nullptr;
     a.rhs = addF ? rhs : nullptr;
     if (!a.val && !a.rhs) return RG_OK;
-    const int grid = (int)((d->n + kRowsPerCta - 1) / kRowsPerCta);
-    if (d->dim == 3 && !reduced && uni)
-        RG_TIMED(T_ASSEMBLE, (k_assemble<3, 8, true><<<grid, kRowsPerCta, 0, stream()>>>(a)));
-    else if (d->dim == 3 && !reduced)
-        RG_TIMED(T_ASSEMBLE, (k_assemble<3, 8, false><<<grid, kRowsPerCta, 0, stream()>>>(a)));
-    else if (d->dim == 3)
-        RG_TIMED(T_ASSEMBLE, (k_assemble<3, 1, false><<<grid, kRowsPerCta, 0, stream()>>>(a)));
-    else if (!reduced && uni)
-        RG_TIMED(T_ASSEMBLE, (k_assemble<2, 4, true><<<grid, kRowsPerCta, 0, stream()>>>(a)));
-    else if (!reduced)
-        RG_TIMED(T_ASSEMBLE, (k_assemble<2, 4, false><<<grid, kRowsPerCta, 0, stream()>>>(a)));
-    else
-        RG_TIMED(T_ASSEMBLE, (k_assemble<2, 1, false><<<grid, kRowsPerCta, 0, stream()>>>(a)));
-    RG_CHECK_LAUNCH();
-    return RG_OK;
+    if (uni) return d->dim == 3 ? launch_assemble_uni<3, 8>(a) : launch_assemble_uni<2, 4>(a);
+    if (d->dim == 3) return reduced ? launch_assemble<3, 1>(a) : launch_assemble<3, 8>(a);
+    return reduced ? launch_assemble<2, 1>(a) : launch_assemble<2, 4>(a);
 }
 
 template <int DIM, bool RED>
