@@ -53,8 +53,8 @@ int coef_begin(Matrix* m)
 {
     CoefRecord& c = m->coef;
     const Domain* d = m->dom;
-    if (!c.khat) RG_CHECK_CUDA(cudaMalloc((void**)&c.khat, sizeof(float) * khat_size(d)));
-    if (!c.bad) RG_CHECK_CUDA(cudaMalloc((void**)&c.bad, sizeof(int)));
+    if (!c.khat) RG_CHECK_CUDA(dev_malloc((void**)&c.khat, sizeof(float) * khat_size(d)));
+    if (!c.bad) RG_CHECK_CUDA(dev_malloc((void**)&c.bad, sizeof(int)));
     RG_CHECK_CUDA(cudaMemsetAsync(c.khat, 0, sizeof(float) * khat_size(d), stream()));
     RG_CHECK_CUDA(cudaMemsetAsync(c.bad, 0, sizeof(int), stream()));
     c.state = 1;
@@ -129,8 +129,8 @@ int coef_usable(Matrix* m, bool* usable)
 
 void free_coef(Matrix* m)
 {
-    if (m->coef.khat) cudaFree(m->coef.khat);
-    if (m->coef.bad) cudaFree(m->coef.bad);
+    if (m->coef.khat) dev_free(m->coef.khat);
+    if (m->coef.bad) dev_free(m->coef.bad);
     m->coef = CoefRecord();
 }
 

@@ -116,6 +116,15 @@ struct Matrix {
     CoefRecord coef;
 };
 
+// ---------------------------------------------------------------- memory (rg_pool.cu)
+// Device blocks from the library's pool on the current device, ordered on stream(); a block is given back
+// after a device synchronisation, as cudaFree implies one.  Pinned host blocks of at most kPinnedBlock bytes.
+cudaError_t dev_malloc(void** p, size_t bytes);
+void dev_free(void* p);
+constexpr size_t kPinnedBlock = 1024;
+cudaError_t pinned_malloc(void** p, size_t bytes);
+void pinned_free(void* p);
+
 // ---------------------------------------------------------------- deterministic reductions
 // Every block writes NV partial sums; the last block to finish (atomic ticket) sums
 // the partials in a fixed order, so results do not depend on block scheduling.

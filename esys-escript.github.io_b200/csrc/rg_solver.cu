@@ -106,7 +106,7 @@ namespace {
 template <typename T>
 int dalloc(T** p, size_t count)
 {
-    RG_CHECK_CUDA(cudaMalloc((void**)p, sizeof(T) * (count ? count : 1)));
+    RG_CHECK_CUDA(dev_malloc((void**)p, sizeof(T) * (count ? count : 1)));
     return RG_OK;
 }
 
@@ -139,8 +139,8 @@ int ensure_workspace(Matrix* m, bool fp32)
             (rc = dalloc(&w->s, 1)) || (rc = dalloc(&w->bad, 1)) ||
             (rc = dalloc((unsigned char**)&w->mail, kMailBytes)))
             return rc;
-        RG_CHECK_CUDA(cudaMallocHost((void**)&w->hs, sizeof(Scal)));
-        RG_CHECK_CUDA(cudaMallocHost((void**)&w->hpoll, 2 * sizeof(Scal)));
+        RG_CHECK_CUDA(pinned_malloc((void**)&w->hs, sizeof(Scal)));
+        RG_CHECK_CUDA(pinned_malloc((void**)&w->hpoll, 2 * sizeof(Scal)));
         RG_CHECK_CUDA(cudaStreamCreateWithFlags(&w->priv, cudaStreamNonBlocking));
         RG_CHECK_CUDA(cudaEventCreateWithFlags(&w->ev_in, cudaEventDisableTiming));
         RG_CHECK_CUDA(cudaEventCreateWithFlags(&w->ev_out, cudaEventDisableTiming));
@@ -1556,7 +1556,7 @@ int run_pcg64_t(Matrix* m, long long cap, long long* iters, int* status)
 int run_pcg64(Matrix* m, bool paso, long long cap, long long* iters, int* status)
 {
     Workspace* w = m->ws;
-    if (!w->p2) RG_CHECK_CUDA(cudaMalloc((void**)&w->p2, sizeof(double) * m->dom->n));
+    if (!w->p2) RG_CHECK_CUDA(dev_malloc((void**)&w->p2, sizeof(double) * m->dom->n));
     if (m->dom->nbands == 27)
         return paso ? run_pcg64_t<27, true>(m, cap, iters, status) : run_pcg64_t<27, false>(m, cap, iters, status);
     return paso ? run_pcg64_t<9, true>(m, cap, iters, status) : run_pcg64_t<9, false>(m, cap, iters, status);
@@ -1925,10 +1925,10 @@ int prepare(Matrix* m, bool want_band, bool want_band64)
     Workspace* w = m->ws;
     // a band copy is written once a solve reads it and kept current from then on; arrays
     // adopted from a destroyed matrix are not written until then
-    if (want_band && !m->band32) RG_CHECK_CUDA(cudaMalloc((void**)&m->band32, sizeof(float) * d->nbands * d->npad));
-    if (want_band && !m->dinv32) RG_CHECK_CUDA(cudaMalloc((void**)&m->dinv32, sizeof(float) * d->n));
+    if (want_band && !m->band32) RG_CHECK_CUDA(dev_malloc((void**)&m->band32, sizeof(float) * d->nbands * d->npad));
+    if (want_band && !m->dinv32) RG_CHECK_CUDA(dev_malloc((void**)&m->dinv32, sizeof(float) * d->n));
     if (want_band64 && !m->band64)
-        RG_CHECK_CUDA(cudaMalloc((void**)&m->band64, sizeof(double) * d->nbands * d->npad));
+        RG_CHECK_CUDA(dev_malloc((void**)&m->band64, sizeof(double) * d->nbands * d->npad));
     if ((want_band && !m->band32_ok) || (want_band64 && !m->band64_ok)) m->solver_ready = false;
     want_band = want_band || m->band32_ok;
     want_band64 = want_band64 || m->band64_ok;
@@ -1937,7 +1937,7 @@ int prepare(Matrix* m, bool want_band, bool want_band64)
         if (rc) return rc;
     }
     if (m->balanced && m->solver_ready) return RG_OK;
-    if (!m->dinv) RG_CHECK_CUDA(cudaMalloc((void**)&m->dinv, sizeof(double) * d->n));
+    if (!m->dinv) RG_CHECK_CUDA(dev_malloc((void**)&m->dinv, sizeof(double) * d->n));
     RG_CHECK_CUDA(cudaMemsetAsync(w->bad, 0, sizeof(int), stream()));
     int rc = launch_balance(m, m->balanced ? 0 : 1, w->bad, want_band, want_band64);
     if (rc) return rc;
@@ -2249,16 +2249,16 @@ void free_workspace(Matrix* m)
     Workspace* w = m->ws;
     if (!w) return;
     double* dd[] = {w->r, w->x, w->rs, w->x2, w->q, w->z, w->p, w->p2, w->bb, w->partials};
-    for (double* p : dd) cudaFree(p);
-    cudaFree(w->mail);
-    cudaFree(w->d32);
-    cudaFree(w->v4[0]);
-    cudaFree(w->v4[1]);
-    cudaFree(w->counter);
-    cudaFree(w->s);
-    cudaFree(w->bad);
-    cudaFreeHost(w->hs);
-    cudaFreeHost(w->hpoll);
+    for (double* p : dd) dev_free(p);
+    dev_free(w->mail);
+    dev_free(w->d32);
+    dev_free(w->v4[0]);
+    dev_free(w->v4[1]);
+    dev_free(w->counter);
+    dev_free(w->s);
+    dev_free(w->bad);
+    pinned_free(w->hs);
+    pinned_free(w->hpoll);
     for (int k = 0; k < 3; ++k)
         if (w->graph[k]) cudaGraphExecDestroy(w->graph[k]);
     if (w->ev_in) cudaEventDestroy(w->ev_in);

@@ -699,12 +699,12 @@ SysWorkspace* ensure_ws(Matrix* m)
     cudaError_t e = cudaSuccess;
     double** v[] = {&w->r, &w->x, &w->rs, &w->x2, &w->q, &w->z, &w->p, &w->bb};
     for (double** pp : v)
-        if (e == cudaSuccess) e = cudaMalloc((void**)pp, sizeof(double) * (N ? N : 1));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&w->partials, sizeof(double) * 4 * kNumSMs * 64);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&w->counter, sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMalloc(&w->s, sizeof(BScal));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&w->bad, sizeof(int));
-    if (e == cudaSuccess) e = cudaMallocHost(&w->hs, sizeof(BScal));
+        if (e == cudaSuccess) e = dev_malloc((void**)pp, sizeof(double) * (N ? N : 1));
+    if (e == cudaSuccess) e = dev_malloc((void**)&w->partials, sizeof(double) * 4 * kNumSMs * 64);
+    if (e == cudaSuccess) e = dev_malloc((void**)&w->counter, sizeof(unsigned));
+    if (e == cudaSuccess) e = dev_malloc(&w->s, sizeof(BScal));
+    if (e == cudaSuccess) e = dev_malloc((void**)&w->bad, sizeof(int));
+    if (e == cudaSuccess) e = pinned_malloc(&w->hs, sizeof(BScal));
     if (e == cudaSuccess) e = cudaMemsetAsync(w->counter, 0, sizeof(unsigned), stream());
     m->sws = w;
     if (e != cudaSuccess) {
@@ -728,7 +728,7 @@ int prepare_sys(Matrix* m, SysWorkspace* w)
 {
     const Domain* d = m->dom;
     if (m->balanced && m->solver_ready) return RG_OK;
-    if (!m->dinv) RG_CHECK_CUDA(cudaMalloc((void**)&m->dinv, sizeof(double) * d->n * NB * NB));
+    if (!m->dinv) RG_CHECK_CUDA(dev_malloc((void**)&m->dinv, sizeof(double) * d->n * NB * NB));
     const int grid = grid_for(d->n * NB, kThreads / kLpr, 16);
     if (!m->balanced) {
         RG_TIMED(T_BALANCE, (k_balance_sys<NB><<<grid, kThreads, 0, stream()>>>(d->n, d->ptr, m->val, m->bv)));
@@ -1048,11 +1048,11 @@ void free_system_workspace(Matrix* m)
     SysWorkspace* w = m->sws;
     if (!w) return;
     double* v[] = {w->r, w->x, w->rs, w->x2, w->q, w->z, w->p, w->bb, w->partials};
-    for (double* p : v) cudaFree(p);
-    cudaFree(w->counter);
-    cudaFree(w->s);
-    cudaFree(w->bad);
-    cudaFreeHost(w->hs);
+    for (double* p : v) dev_free(p);
+    dev_free(w->counter);
+    dev_free(w->s);
+    dev_free(w->bad);
+    pinned_free(w->hs);
     delete w;
     m->sws = nullptr;
 }
