@@ -324,7 +324,7 @@ int rg_matrix_create_system(rg_domain* dom, int block_size, rg_matrix** out)
     m.dom = &dom->d;
     m.nb = block_size;
     const size_t nv = (size_t)dom->d.nnz * block_size * block_size;
-    cudaError_t e = dev_malloc((void**)&m.val, sizeof(double) * nv);
+    cudaError_t e = dev_malloc((void**)&m.val, sizeof(double) * (nv + 2));  // (as above)
     if (e == cudaSuccess) e = dev_malloc((void**)&m.bv, sizeof(double) * dom->d.n * block_size);
     if (e == cudaSuccess) e = cudaMemsetAsync(m.val, 0, sizeof(double) * nv, stream());
     if (e != cudaSuccess) {
@@ -600,8 +600,8 @@ int rg_solver_set_config(rg_matrix* mat, int spmv_config)
 
 int rg_test_wait_limit(int max_polls, int withhold_copies)
 {
-    const int rc = rg::set_wait_control(max_polls, withhold_copies);
-    if (rc) return rc;
+    int rc = rg::set_wait_control(max_polls, withhold_copies);
+    if (rc || (rc = rg::sys::set_wait_control(max_polls, withhold_copies))) return rc;
     return rg::ws::set_conv_wait_control(max_polls, withhold_copies);
 }
 

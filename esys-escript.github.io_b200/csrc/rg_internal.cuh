@@ -274,6 +274,9 @@ namespace ws {
 // the same test hook for the persistent convolution (ws_conv.cu)
 int set_conv_wait_control(int polls, int withhold);
 }  // namespace ws
+namespace sys {
+int set_wait_control(int polls, int withhold);  // and for the block PCG (rg_system.cu)
+}  // namespace sys
 void free_workspace(Matrix* m);
 // hands the matrix's solver vectors to its domain for the next matrix there (one is kept; a
 // further one is freed), instead of freeing them: a fresh matrix on the same grid then

@@ -22,13 +22,6 @@
 // 200 x 200 paso 5.9 against 20 us, 403 x 297 textbook 6.4 against 15 us.
 #pragma once
 
-// Scalars of one CTA's copy of the iteration (all CTAs compute the same values)
-struct Pcg64State {
-    double alpha, beta, g1, g2, tau, tau_next, rho, delta, norm;
-    long long iter;
-    int status, stop;
-};
-
 struct Pcg64Args {
     int n, nn0, nn1, nn2;
     int off[27];                  // column offset of band b
@@ -47,19 +40,6 @@ template <int NB, int W, int S>
 constexpr size_t pcg64_smem()
 {
     return (size_t)W * S * (32 * NB * 8 + 16);
-}
-
-__host__ inline void fast_div(unsigned d, unsigned* m, int* s)
-{
-    int k = 0;
-    while ((1ull << k) < d) ++k;
-    *s = k;
-    *m = (unsigned)((1ull << (31 + k)) / d + 1);
-}
-
-__device__ __forceinline__ unsigned fdiv(unsigned v, unsigned m, int s)
-{
-    return (unsigned)(((unsigned long long)v * m) >> (31 + s));
 }
 
 template <int NB, int W, int S, bool PASO>
@@ -85,7 +65,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
         sc.rho = s->rho;
         sc.norm = s->norm;
         sc.iter = s->iter;
-        sc.status = ST_RUN;
+        sc.status = PCG_RUN;
         sc.stop = 0;
     }
     if (threadIdx.x < W * S) mbar_init(&full[threadIdx.x / S][threadIdx.x % S], 1);
@@ -252,28 +232,17 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
         bool ok = mail_sum<2, W, false>(v, t, a.mail, gen, &bad, polls, wc.withhold != 0);
         if (threadIdx.x == 0) {
             if (!ok) {
-                sc.status = ST_TIMEOUT;
+                sc.status = PCG_TIMEOUT;
                 sc.stop = 1;
             } else {
-                if (PASO && pend) {
-                    // the iteration before is complete: its stopping tests (PCG.cpp:307-347)
-                    sc.iter += 1;
-                    sc.norm = sqrt(t[1]);
-                    if (sc.iter > maxit)
-                        sc.status = ST_MAXIT;
-                    else if (fabs(sc.tau) <= 0.0)
-                        sc.status = ST_BREAK;
-                    else if (sc.norm <= tol)
-                        sc.status = ST_CONV;
-                    sc.tau = sc.tau_next;
-                    if (sc.status != ST_RUN) sc.stop = 1;
-                }
-                if (!sc.stop) {
+                if (PASO) {
+                    paso_after_a(sc, t, pend, tol, maxit);
+                } else {
                     sc.delta = t[0];
-                    sc.alpha = (PASO ? sc.tau : sc.rho) / t[0];
-                    if (PASO ? fabs(t[0]) <= 0.0 : !(fabs(t[0]) > 0.0)) {  // breakFlag (PCG.cpp:228-262)
+                    sc.alpha = sc.rho / t[0];
+                    if (!(fabs(t[0]) > 0.0)) {
                         sc.iter += 1;
-                        sc.status = ST_BREAK;
+                        sc.status = PCG_BREAK;
                         sc.stop = 1;
                     }
                 }
@@ -311,13 +280,10 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
         ok = mail_sum<3, W, true>(u, w, a.mail, gen, &bad, polls, wc.withhold != 0);
         if (threadIdx.x == 0) {
             if (!ok) {
-                sc.status = ST_TIMEOUT;
+                sc.status = PCG_TIMEOUT;
                 sc.stop = 1;
             } else if (PASO) {
-                sc.g1 = fabs(w[1]) <= 0.0 ? 0.0 : -w[2] / w[1];
-                sc.g2 = 1.0 - sc.g1;
-                sc.tau_next = w[0];
-                sc.beta = w[0] / sc.tau;
+                paso_after_b(sc, w);
                 if (left == 1) sc.stop = 1;
             } else {
                 sc.iter += 1;
@@ -325,12 +291,12 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
                 sc.beta = w[0] / sc.rho;
                 sc.rho = w[0];
                 if (sc.norm <= tol)
-                    sc.status = ST_CONV;
+                    sc.status = PCG_CONV;
                 else if (sc.iter >= maxit)
-                    sc.status = ST_MAXIT;
+                    sc.status = PCG_MAXIT;
                 else if (!(fabs(w[0]) > 0.0))
-                    sc.status = ST_BREAK;
-                if (sc.status != ST_RUN || left == 1) sc.stop = 1;
+                    sc.status = PCG_BREAK;
+                if (sc.status != PCG_RUN || left == 1) sc.stop = 1;
             }
         }
         __syncthreads();
@@ -344,8 +310,8 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
             mbar_wait(&full[warp][k % S], (uint32_t)((k / S) & 1));
     }
     if (threadIdx.x == 0) {
-        if (sc.status == ST_TIMEOUT) {
-            report_status(s, ST_TIMEOUT);
+        if (sc.status == PCG_TIMEOUT) {
+            report_status(s, PCG_TIMEOUT);
         } else if (blockIdx.x == 0) {
             s->alpha = sc.alpha;
             s->beta = sc.beta;
@@ -359,7 +325,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
             s->iter = sc.iter;
             s->par = par;
             s->pend = pend ? 1 : 0;
-            if (sc.status != ST_RUN) report_status(s, sc.status);
+            if (sc.status != PCG_RUN) report_status(s, sc.status);
         }
     }
 }

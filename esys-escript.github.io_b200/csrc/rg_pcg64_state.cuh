@@ -1,0 +1,69 @@
+// What the persistent FP64 PCG kernels share (rg_pcg64.cuh for scalar matrices, rg_system.cu for block
+// ones): a CTA's copy of the iteration's scalars, paso's scalar steps (PCG.cpp:185-347), and division of
+// node numbers by the grid's sizes.
+#pragma once
+#include <cstdint>
+
+namespace rg {
+
+// iteration status, as in the solvers' device scalars
+enum { PCG_RUN = 0, PCG_CONV = 1, PCG_MAXIT = 3, PCG_BREAK = 4, PCG_TIMEOUT = 6 };
+
+struct Pcg64State {  // (all CTAs compute the same values)
+    double alpha, beta, g1, g2, tau, tau_next, rho, delta, norm;
+    long long iter;
+    int status, stop;
+};
+
+// After the product: t = {p.v, |rs|^2}.  With `pend` the iteration before is complete: its stopping tests;
+// then alpha = tau / delta, breakdown on delta == 0.
+__device__ __forceinline__ void paso_after_a(Pcg64State& sc, const double* t, bool pend, double tol, long long maxit)
+{
+    if (pend) {
+        sc.iter += 1;
+        sc.norm = sqrt(t[1]);
+        if (sc.iter > maxit)
+            sc.status = PCG_MAXIT;
+        else if (fabs(sc.tau) <= 0.0)
+            sc.status = PCG_BREAK;
+        else if (sc.norm <= tol)
+            sc.status = PCG_CONV;
+        sc.tau = sc.tau_next;
+        if (sc.status != PCG_RUN) {
+            sc.stop = 1;
+            return;
+        }
+    }
+    sc.delta = t[0];
+    sc.alpha = sc.tau / t[0];
+    if (fabs(t[0]) <= 0.0) {  // breakFlag
+        sc.iter += 1;
+        sc.status = PCG_BREAK;
+        sc.stop = 1;
+    }
+}
+
+// After the update: w = {z.r, d.d, d.rs} with d = r - rs: the smoothing weights and the next beta.
+__device__ __forceinline__ void paso_after_b(Pcg64State& sc, const double* w)
+{
+    sc.g1 = fabs(w[1]) <= 0.0 ? 0.0 : -w[2] / w[1];
+    sc.g2 = 1.0 - sc.g1;
+    sc.tau_next = w[0];
+    sc.beta = w[0] / sc.tau;
+}
+
+// v / d = (v m) >> (31 + s) for v < 2^31
+inline void fast_div(unsigned d, unsigned* m, int* s)
+{
+    int k = 0;
+    while ((1ull << k) < d) ++k;
+    *s = k;
+    *m = (unsigned)((1ull << (31 + k)) / d + 1);
+}
+
+__device__ __forceinline__ unsigned fdiv(unsigned v, unsigned m, int s)
+{
+    return (unsigned)(((unsigned long long)v * m) >> (31 + s));
+}
+
+}  // namespace rg

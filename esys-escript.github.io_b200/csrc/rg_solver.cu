@@ -33,6 +33,7 @@
 #include "rg_bulk.cuh"
 #include "rg_gridmail.cuh"
 #include "rg_internal.cuh"
+#include "rg_pcg64_state.cuh"
 
 namespace rg {
 using namespace bulk;
