@@ -21,9 +21,10 @@
 
 namespace rg {
 
-constexpr int kMailCtas = 160;      // most CTAs of a grid that exchanges (5 per lane of a warp)
+constexpr int kMailCtas = 160;      // CTAs whose posts a warp reads at a time (5 per lane)
+constexpr int kMailGrid = 2 * kMailCtas;  // most CTAs of a grid that exchanges with SYNC; else kMailCtas
 constexpr int kMailVals = 8;        // most doubles of an exchange
-constexpr size_t kMailSet = (size_t)2 * kMailVals * kMailCtas;  // 8-byte words of one set
+constexpr size_t kMailSet = (size_t)2 * kMailVals * kMailCtas;  // 8-byte words of one set (kMailVals x kMailGrid with SYNC)
 constexpr size_t kMailBytes = 8 * (2 * kMailSet + 16);
 constexpr unsigned kMailAbort = 0x80000000u;
 
@@ -103,7 +104,7 @@ __device__ __forceinline__ bool mail_sum(const double (&v)[NV], double (&tot)[NV
     const unsigned long long tag = (unsigned long long)gen << 32;
     const int G = (int)gridDim.x;
     if (SYNC) {
-        if (sub == 0 && val < NV) mail_store(set + val * kMailCtas + blockIdx.x, bits);
+        if (sub == 0 && val < NV) mail_store(set + val * kMailGrid + blockIdx.x, bits);
     } else if (sub < 2 && val < NV) {
         mail_store(set + (2 * val + sub) * kMailCtas + blockIdx.x, tag | (sub ? bits >> 32 : bits & 0xffffffffull));
     }
@@ -133,16 +134,18 @@ __device__ __forceinline__ bool mail_sum(const double (&v)[NV], double (&tot)[NV
 #pragma unroll
     for (int j = 0; j < P; ++j) part[j] = 0.0;
     if (SYNC) {
-        unsigned long long w[K][NV];
+        for (int first = 0; first < G; first += kMailCtas) {
+            unsigned long long w[K][NV];
 #pragma unroll
-        for (int k = 0; k < K; ++k)
+            for (int k = 0; k < K; ++k)
+#pragma unroll
+                for (int j = 0; j < NV; ++j)
+                    w[k][j] = first + lane + 32 * k < G ? mail_load(set + j * kMailGrid + first + lane + 32 * k) : 0ull;
 #pragma unroll
             for (int j = 0; j < NV; ++j)
-                w[k][j] = lane + 32 * k < G ? mail_load(set + j * kMailCtas + lane + 32 * k) : 0ull;
 #pragma unroll
-        for (int j = 0; j < NV; ++j)
-#pragma unroll
-            for (int k = 0; k < K; ++k) part[j] += __longlong_as_double((long long)w[k][j]);
+                for (int k = 0; k < K; ++k) part[j] += __longlong_as_double((long long)w[k][j]);
+        }
     } else {
         for (;; ++tries) {
             unsigned long long w[K][2 * NV];

@@ -10,8 +10,8 @@
 //    recursive FP32 residual has dropped by `inner_tolerance` the true residual is
 //    recomputed in FP64 on the CSR values, tested with paso's dual-norm criterion and
 //    written back into the FP32 recurrence (the Krylov direction is kept, no restart).
-//    One FP32 iteration is one kernel (k_f32_cg, the one-reduction recurrence of
-//    Chronopoulos and Gear).
+//    (k_f32_cg, k_f32_cg_coef: the one-reduction recurrence of Chronopoulos and Gear, many
+//    iterations per launch).
 //
 // FP64 PCG runs in one persistent kernel over many iterations (rg_pcg64.cuh).  With more than
 // one Jacobi sweep (paso mode) an iteration is a kernel per step instead: a pure SpMV of the
@@ -775,7 +775,7 @@ constexpr int band64_stages() { return NB == 27 ? 3 : 8; }
 
 #include "rg_pcg64.cuh"
 
-// ------------------------------------------------------------------ FP32 PCG, one kernel per iteration
+// ------------------------------------------------------------------ FP32 PCG, one reduction per iteration
 // Jacobi-PCG in the one-reduction form of Chronopoulos and Gear ("s-step iterative methods
 // for symmetric linear systems", J. Comput. Appl. Math. 25, 1989): besides the search
 // direction p the recurrences carry s = A p and w = A u (u = D^-1 r, the preconditioned
@@ -803,8 +803,12 @@ constexpr int band64_stages() { return NB == 27 ? 3 : 8; }
 // consumer thread forms u_{i+1} once per stencil column, at its own dx = 0 position, and takes
 // the dx = -1 / +1 values from the neighbouring lanes (warp shuffles; lanes 0 and 31 form their
 // outer neighbour themselves): 9 state loads per row instead of 27.  Per row the kernel moves
-// the 108 band bytes, 16 bytes of state in and out and the correction d (8 bytes): 148 B, in
-// one launch with one reduction.
+// the 108 band bytes, 16 bytes of state in and out and the correction d (8 bytes): 148 B.
+//
+// A launch runs many iterations; one grid-wide exchange of the six sums (rg_gridmail.cuh) ends each,
+// and the band blocks of the next iteration's first tiles are copied while it waits.  Against a launch
+// and a reduction by the last CTA per iteration: 10.6 against 15 us at 64^3, 20.7 against 25.2 us at
+// 96 x 113 x 82.
 //
 // mode 0: iteration.  mode 1/2: start of a segment (fresh / continuing direction): u was just
 // seeded from the FP64 residual; both A u and A p_prev are formed from the windows (no
@@ -921,175 +925,218 @@ __device__ void cg_scalars(Scal* s, const double* tt, int mode)
 // is bulk-copied with the state windows; the diagonal is its centre band.
 template <int NB, int kStages, int kCtas>
 __global__ void __launch_bounds__(kTile + 32, kCtas) k_f32_cg(const float* __restrict__ band,
-                                                              const __grid_constant__ CgArgs ca,
-                                                              const float4* V0, const float4* V1,
-                                                              float4* W0, float4* W1,
-                                                              float* __restrict__ d, ReduceBuf rb, Scal* s, int mode)
+                                                              const __grid_constant__ CgArgs ca, float4* V0, float4* V1,
+                                                              float* d, unsigned long long* mail, Scal* s, int mode,
+                                                              int max_iters)
 {
     constexpr int kCenter = NB / 2;
     constexpr int NG = NB / 3;
+    constexpr int W = kConsumerWarps + 1;
     extern __shared__ __align__(128) float smem[];
     __shared__ __align__(8) uint64_t full[kStages], empty[kStages];
+    __shared__ Scal sc;
     __shared__ int bad;
     if (mode == 0 && s->done) return;
-    const float alpha = mode == 0 ? (float)s->alpha : 0.f;
-    const float beta = mode == 0 ? (float)s->beta : 0.f;
-    const bool odd = (s->pk & 1) != 0;
-    const float4* __restrict__ vin = odd ? V1 : V0;   // state of this iteration
-    float4* __restrict__ vout = odd ? W0 : W1;        // state of the next one
     const int t = threadIdx.x;
     const int lane = t & 31;
     const int warp = t >> 5;
     const int eoff = lane == 0 ? -1 : (lane == 31 ? 1 : 0);  // the outer x-neighbour of warp edge lanes
     const int64_t n = ca.n;
     const int64_t ntiles = (n + kTile - 1) / kTile;
-    const int64_t my_tiles = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-    // tile k of this CTA; odd iterations walk the tiles backwards, so that the state rows the
-    // previous launch wrote last, the likeliest to be still in L2, are read first (measured at
-    // 128^3: 58.4 -> 55.4 us per launch)
-    const bool back = odd;
-    const int64_t tbase = back ? ntiles - 1 - blockIdx.x : (int64_t)blockIdx.x;
-    const int64_t tstep = back ? -(int64_t)gridDim.x : (int64_t)gridDim.x;
-    auto tile_of = [&](int64_t k) { return tbase + k * tstep; };
+    const int my_tiles = blockIdx.x < ntiles ? (int)((ntiles - 1 - blockIdx.x) / gridDim.x) + 1 : 0;
     constexpr int kmat = NB * kTile;  // floats of the operator's part of a stage
     const int stage_floats = kmat + 4 * ca.nwin * ca.wlen;
+    const uint32_t wbytes = (uint32_t)ca.wlen * 16u;
     if (t == 0) {
         for (int k = 0; k < kStages; ++k) {
             mbar_init(&full[k], 1);
             mbar_init(&empty[k], kConsumerWarps);
         }
         bad = 0;
+        sc = *s;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
     auto interior = [&](int64_t i0) { return i0 + ca.lo >= 0 && i0 + ca.hi <= n; };
-
-    // sums: g = r.u, |r|^2, u.w, u.s, p.w, p.s (u, w of the next iteration; p, s of this one)
-    double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    int64_t issued = 0;
+    // tile k of this CTA; odd iterations walk the tiles backwards, so that the state rows the iteration
+    // before wrote last, the likeliest to be still in L2, are read first (measured at 128^3: 58.4 ->
+    // 55.4 us per iteration)
+    auto tile_of = [&](int k, bool back) {
+        const int64_t b = back ? ntiles - 1 - blockIdx.x : (int64_t)blockIdx.x;
+        return b + (back ? -(int64_t)k : (int64_t)k) * gridDim.x;
+    };
     const WaitCtl wc = g_wait_ctl;
     const int polls = wc.polls > 0 ? wc.polls : kDefaultPolls;
-    if (warp == kConsumerWarps) {
-        // ---------------- producer: operator data and state windows of each tile
-        if (lane == 0 && !wc.withhold) {
-            const uint64_t pol = evict_first_policy();
-            const uint32_t wbytes = (uint32_t)ca.wlen * 16u;
-            for (int64_t k = 0; k < my_tiles; ++k, issued = k) {
-                const int st = (int)(k % kStages);
-                if (k >= kStages && !mbar_wait(&empty[st], (uint32_t)(((k / kStages) - 1) & 1), polls)) {
+    const uint64_t pol = evict_first_policy();
+    int64_t issued = 0;               // producer: tiles whose band copies were issued, over all iterations
+    int64_t base = 0;                 // tiles of the iterations before
+    unsigned gen = 0;
+    bool failed = false;
+    // producer: the stage of running tile c, tile k of an iteration: its band block; false: a wait gave up
+    auto issue_band = [&](int64_t c, int k, bool back) {
+        const int st = (int)(c % kStages);
+        if (c >= kStages && !mbar_wait(&empty[st], (uint32_t)(((c / kStages) - 1) & 1), polls)) return false;
+        const int64_t tile = tile_of(k, back);
+        const bool in = interior(tile * kTile);
+        mbar_expect_tx(&full[st], (uint32_t)kmat * 4u + (in ? (uint32_t)ca.nwin * wbytes : 0u));
+        bulk_g2s_hint(smem + (size_t)st * stage_floats, band + (size_t)tile * NB * kTile, NB * kTile * 4, &full[st], pol);
+        issued = c + 1;
+        return true;
+    };
+    for (int it = 0; it < max_iters; ++it) {
+        const float alpha = mode == 0 ? (float)sc.alpha : 0.f;
+        const float beta = mode == 0 ? (float)sc.beta : 0.f;
+        const bool odd = (sc.pk & 1) != 0;
+        const float4* vin = odd ? V1 : V0;   // state of this iteration
+        float4* vout = odd ? V0 : V1;        // state of the next one
+        // sums: g = r.u, |r|^2, u.w, u.s, p.w, p.s (u, w of the next iteration; p, s of this one)
+        double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        if (warp == kConsumerWarps) {
+            // ---------------- producer: operator data and state windows of each tile; the first tiles'
+            // band blocks of the next iteration are issued before this one's exchange (they are not new)
+            if (lane == 0 && !wc.withhold) {
+                for (int k = 0; k < my_tiles && !failed; ++k) {
+                    const int64_t c = base + k;
+                    if (issued <= c && !issue_band(c, k, odd)) {
+                        failed = true;
+                        break;
+                    }
+                    const int st = (int)(c % kStages);
+                    const int64_t i0 = tile_of(k, odd) * kTile;
+                    if (interior(i0))
+                        for (int w = 0; w < ca.nwin; ++w)
+                            bulk_g2s(smem + (size_t)st * stage_floats + kmat + 4 * w * ca.wlen, vin + (i0 + ca.woff[w]),
+                                     wbytes, &full[st]);
+                }
+                if (it + 1 < max_iters)
+                    for (int k = 0; k < kStages && k < my_tiles && !failed; ++k)
+                        failed = !issue_band(base + my_tiles + k, k, !odd);
+                if (failed) bad = 1;
+            }
+        } else {
+            // ---------------- consumers: row i0 + t of every tile
+            for (int k = 0; k < my_tiles; ++k) {
+                const int64_t c = base + k;
+                const int st = (int)(c % kStages);
+                const int64_t i0 = tile_of(k, odd) * (int64_t)kTile;
+                const int64_t i = i0 + t;
+                // the correction is only read and written by this row: load it while the stage fills
+                const float dold = (mode == 0 && i < n) ? __ldcs(d + i) : 0.f;
+                if (!mbar_wait(&full[st], (uint32_t)((c / kStages) & 1), polls)) {
                     bad = 1;
                     break;
                 }
-                const int64_t tile = tile_of(k);
-                const int64_t i0 = tile * kTile;
-                float* dst = smem + (size_t)st * stage_floats;
-                const bool in = interior(i0);
-                mbar_expect_tx(&full[st], (uint32_t)kmat * 4u + (in ? (uint32_t)ca.nwin * wbytes : 0u));
-                bulk_g2s_hint(dst, band + (size_t)tile * NB * kTile, NB * kTile * 4, &full[st], pol);
-                if (in)
-                    for (int w = 0; w < ca.nwin; ++w)
-                        bulk_g2s(dst + kmat + 4 * w * ca.wlen, vin + (i0 + ca.woff[w]), wbytes, &full[st]);
-            }
-        }
-    } else {
-        // ---------------- consumers: row i0 + t of every tile
-        for (int k = 0; k < (int)my_tiles; ++k) {  // (32-bit tile count: cheaper stage arithmetic)
-            const int st = k % kStages;
-            const int64_t i0 = tile_of(k) * (int64_t)kTile;
-            const int64_t i = i0 + t;
-            // the correction is only read and written by this row: load it while the stage fills
-            const float dold = (mode == 0 && i < n) ? __ldcs(d + i) : 0.f;
-            if (!mbar_wait(&full[st], (uint32_t)((k / kStages) & 1), polls)) {
-                bad = 1;
-                break;
-            }
-            const float* bs = smem + st * stage_floats;
-            const float4* win = reinterpret_cast<const float4*>(bs + kmat);
-            auto coefb = [&](int b) -> float { return bs[b * kTile + t]; };
-            float acc_u = 0.f, acc_p = 0.f;
-            float4 c = make_float4(0.f, 0.f, 0.f, 0.f);  // this row's state
-            if (interior(i0) && mode == 0) {
+                const float* bs = smem + st * stage_floats;
+                const float4* win = reinterpret_cast<const float4*>(bs + kmat);
+                auto coefb = [&](int b) -> float { return bs[b * kTile + t]; };
+                float acc_u = 0.f, acc_p = 0.f;
+                float4 cst = make_float4(0.f, 0.f, 0.f, 0.f);  // this row's state
+                if (interior(i0) && mode == 0) {
 #pragma unroll
-                for (int g = 0; g < NG; ++g) {
-                    // u_{i+1} at this lane's dx = 0 neighbour of stencil column g; dx = -1 / +1
-                    // from the lanes beside it; lanes 0 / 31 form that outer value themselves
-                    const int pc = ca.bpos[3 * g + 1] + t;
-                    const float4 vc = win[pc];
-                    const float uc = next_u(vc, alpha, beta);
-                    float ue = 0.f;
-                    if (lane == 0 || lane == 31) ue = next_u(win[pc + eoff], alpha, beta);
-                    const float up = __shfl_up_sync(0xffffffffu, uc, 1);
-                    const float dn = __shfl_down_sync(0xffffffffu, uc, 1);
-                    const float ul = lane == 0 ? ue : up;
-                    const float ur = lane == 31 ? ue : dn;
-                    acc_u = fmaf(coefb(3 * g), ul, acc_u);
-                    acc_u = fmaf(coefb(3 * g + 1), uc, acc_u);
-                    acc_u = fmaf(coefb(3 * g + 2), ur, acc_u);
-                    if (3 * g + 1 == kCenter) c = vc;
-                }
-            } else {
-                const bool in = interior(i0);
-#pragma unroll
-                for (int b = 0; b < NB; ++b) {
-                    float4 nb;
-                    if (in) {
-                        nb = win[ca.bpos[b] + t];
-                    } else {
-                        const int64_t j = min(max(i + ca.off[b], (int64_t)0), n - 1);
-                        nb = __ldg(vin + j);
+                    for (int g = 0; g < NG; ++g) {
+                        // u_{i+1} at this lane's dx = 0 neighbour of stencil column g; dx = -1 / +1
+                        // from the lanes beside it; lanes 0 / 31 form that outer value themselves
+                        const int pc = ca.bpos[3 * g + 1] + t;
+                        const float4 vc = win[pc];
+                        const float uc = next_u(vc, alpha, beta);
+                        float ue = 0.f;
+                        if (lane == 0 || lane == 31) ue = next_u(win[pc + eoff], alpha, beta);
+                        const float up = __shfl_up_sync(0xffffffffu, uc, 1);
+                        const float dn = __shfl_down_sync(0xffffffffu, uc, 1);
+                        const float ul = lane == 0 ? ue : up;
+                        const float ur = lane == 31 ? ue : dn;
+                        acc_u = fmaf(coefb(3 * g), ul, acc_u);
+                        acc_u = fmaf(coefb(3 * g + 1), uc, acc_u);
+                        acc_u = fmaf(coefb(3 * g + 2), ur, acc_u);
+                        if (3 * g + 1 == kCenter) cst = vc;
                     }
-                    if (mode == 0) {
-                        acc_u = fmaf(coefb(b), next_u(nb, alpha, beta), acc_u);
-                    } else {
-                        acc_u = fmaf(coefb(b), nb.x, acc_u);
-                        acc_p = fmaf(coefb(b), nb.w, acc_p);
-                    }
-                    if (b == kCenter) c = nb;
-                }
-            }
-            const float diag = coefb(kCenter);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[st]);
-            if (i < n) {
-                float un, spn, pn;
-                if (mode == 0) {
-                    pn = fmaf(beta, c.w, c.x);      // p_i = u_i + beta p_{i-1}
-                    spn = fmaf(beta, c.z, c.y);     // D^-1 s_i = D^-1 w_i + beta D^-1 s_{i-1}
-                    un = fmaf(-alpha, spn, c.x);    // u_{i+1}, as next_u forms it
-                    d[i] = fmaf(alpha, pn, dold);   // d += alpha p_i
                 } else {
-                    pn = c.w;                       // the kept direction (0 when fresh)
-                    spn = __fdividef(acc_p, diag);  // D^-1 A p, formed afresh
-                    un = c.x;
+                    const bool in = interior(i0);
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        float4 nb;
+                        if (in) {
+                            nb = win[ca.bpos[b] + t];
+                        } else {
+                            const int64_t j = min(max(i + ca.off[b], (int64_t)0), n - 1);
+                            nb = __ldcg(vin + j);
+                        }
+                        if (mode == 0) {
+                            acc_u = fmaf(coefb(b), next_u(nb, alpha, beta), acc_u);
+                        } else {
+                            acc_u = fmaf(coefb(b), nb.x, acc_u);
+                            acc_p = fmaf(coefb(b), nb.w, acc_p);
+                        }
+                        if (b == kCenter) cst = nb;
+                    }
                 }
-                const float w = acc_u;              // (A u_{i+1})_i
-                vout[i] = make_float4(un, __fdividef(w, diag), spn, pn);
-                const double du = un, dd = diag, ds = (double)spn * dd;
-                v[0] += dd * du * du;
-                v[1] += (dd * du) * (dd * du);  // the segment's stopping norm: |r|^2 of the balanced residual
-                v[2] += du * (double)w;
-                v[3] += du * ds;
-                v[4] += (double)pn * (double)w;
-                v[5] += (double)pn * ds;
+                const float diag = coefb(kCenter);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&empty[st]);
+                if (i < n) {
+                    float un, spn, pn;
+                    if (mode == 0) {
+                        pn = fmaf(beta, cst.w, cst.x);   // p_i = u_i + beta p_{i-1}
+                        spn = fmaf(beta, cst.z, cst.y);  // D^-1 s_i = D^-1 w_i + beta D^-1 s_{i-1}
+                        un = fmaf(-alpha, spn, cst.x);   // u_{i+1}, as next_u forms it
+                        d[i] = fmaf(alpha, pn, dold);    // d += alpha p_i
+                    } else {
+                        pn = cst.w;                      // the kept direction (0 when fresh)
+                        spn = __fdividef(acc_p, diag);   // D^-1 A p, formed afresh
+                        un = cst.x;
+                    }
+                    const float w = acc_u;               // (A u_{i+1})_i
+                    vout[i] = make_float4(un, __fdividef(w, diag), spn, pn);
+                    const double du = un, dd = diag, ds = (double)spn * dd;
+                    v[0] += dd * du * du;
+                    v[1] += (dd * du) * (dd * du);  // the segment's stopping norm: |r|^2 of the balanced residual
+                    v[2] += du * (double)w;
+                    v[3] += du * ds;
+                    v[4] += (double)pn * (double)w;
+                    v[5] += (double)pn * ds;
+                }
             }
         }
+        // rows are written by plain stores and read by bulk copies: order the two kinds of access on both
+        // sides of the exchange
+        asm volatile("fence.proxy.async.global;" ::: "memory");
+        double tt[6];
+        ++gen;
+        const bool ok = mail_sum<6, W, true>(v, tt, mail, gen, &bad, polls, wc.withhold != 0);
+        if (t == 0) {
+            if (!ok)
+                report_status(&sc, ST_TIMEOUT);
+            else
+                cg_scalars(&sc, tt, mode);
+        }
+        __syncthreads();
+        asm volatile("fence.proxy.async.global;" ::: "memory");
+        base += my_tiles;
+        if (sc.status == ST_TIMEOUT || (mode == 0 && sc.done)) break;
     }
-    __syncthreads();
-    if (bad) {
-        // let the copies this CTA issued land (bounded) before its shared memory is released
-        if (warp == kConsumerWarps && lane == 0)
-            for (int64_t k = issued > kStages ? issued - kStages : 0; k < issued; ++k)
-                for (int tries = 0; tries < (1 << 20) && !mbar_try_wait(&full[k % kStages], (uint32_t)((k / kStages) & 1));
-                     ++tries) {
-                }
-        if (t == 0) report_status(s, ST_TIMEOUT);
-        // the CTA still takes its turn in the grid reduction (with nothing to add)
-#pragma unroll
-        for (int j = 0; j < 6; ++j) v[j] = 0.0;
+    // copies this CTA issued and nobody waited for land (bounded) before its shared memory is released: band
+    // blocks of an iteration that did not run (their windows were never issued: only the band's bytes are
+    // in flight, and the barrier stays short of them, so the wait is on the copy itself)
+    if (warp == kConsumerWarps && lane == 0 && issued > base) {
+        for (int64_t c = base; c < issued; ++c) {
+            const int st = (int)(c % kStages);
+            const int64_t i0 = tile_of((int)(c - base), (sc.pk & 1) != 0) * kTile;
+            // the windows' share of the bytes, so that the phase can complete
+            if (interior(i0))
+                for (int w = 0; w < ca.nwin; ++w)
+                    bulk_g2s(smem + (size_t)st * stage_floats + kmat + 4 * w * ca.wlen, V0 + (i0 + ca.woff[w]), wbytes,
+                             &full[st]);
+        }
+        for (int64_t c = base; c < issued; ++c)
+            for (int tries = 0; tries < (1 << 20) && !mbar_try_wait(&full[c % kStages], (uint32_t)((c / kStages) & 1));
+                 ++tries) {
+            }
     }
-    double tt[6];
-    if (grid_reduce<6>(v, rb, tt) && threadIdx.x == 0) {
-        cg_scalars(s, tt, mode);
+    if (t == 0) {
+        if (sc.status == ST_TIMEOUT)
+            report_status(s, ST_TIMEOUT);
+        else if (blockIdx.x == 0)
+            *s = sc;
     }
 }
 
@@ -1717,34 +1764,32 @@ bool cg_config_fits(const Domain* d, int cfg, bool coef)
     return blocks >= kSpmvCfg[cfg][1];
 }
 
-// one launch of the fused FP32 iteration on the band copy (mode 0) or of a segment start (mode 1, 2)
+// one launch of up to `iters` FP32 iterations on the band copy (mode 0), or a segment start (mode 1, 2)
 template <int NB, int S, int CPS>
-void launch_cg_k(Matrix* m, const CgArgs& ca, int grid, size_t smem, int mode)
-{
-    Workspace* w = m->ws;
-    RG_TIMED(T_F32_SPMV, (k_f32_cg<NB, S, CPS><<<grid, kTile + 32, smem, stream()>>>(
-                             m->band32, ca, w->v4[0], w->v4[1], w->v4[0], w->v4[1], w->d32, rbuf(w), w->s, mode)));
-}
-
-template <int NB>
-int launch_cg(Matrix* m, int cfg, int mode)
+int launch_band_t(Matrix* m, int mode, int iters)
 {
     const Domain* d = m->dom;
-    const CgArgs ca = cg_args(d);
+    Workspace* w = m->ws;
+    CgArgs ca = cg_args(d);
     const int64_t ntiles = (d->n + kTile - 1) / kTile;
-    const int grid = (int)std::min<int64_t>(ntiles, (int64_t)sm_count() * kSpmvCfg[cfg][1]);
-    const size_t smem = cg_smem(d, ca, kSpmvCfg[cfg][0]);
-    if (cfg == 0)
-        launch_cg_k<NB, 3, 1>(m, ca, grid, smem, mode);
-    else
-        launch_cg_k<NB, 2, 2>(m, ca, grid, smem, mode);
-    RG_CHECK_LAUNCH();
+    const int grid = (int)std::min<int64_t>(ntiles, std::min(sm_count() * CPS, kMailGrid));
+    const size_t smem = cg_smem(d, ca, S);
+    RG_CHECK_CUDA(cudaMemsetAsync(w->mail, 0, kMailBytes, stream()));
+    const float* band = m->band32;
+    float4 *v0 = w->v4[0], *v1 = w->v4[1];
+    void* args[] = {&band, &ca, &v0, &v1, &w->d32, &w->mail, &w->s, &mode, &iters};
+    cudaError_t e;
+    RG_TIMED(T_F32_SPMV, (e = cudaLaunchCooperativeKernel((const void*)k_f32_cg<NB, S, CPS>, dim3(grid), dim3(kTile + 32),
+                                                          args, smem, stream())));
+    RG_CHECK_CUDA(e);
     return RG_OK;
 }
 
-int launch_band_cfg(Matrix* m, int cfg, int mode = 0)
+int launch_band_cfg(Matrix* m, int cfg, int mode, int iters)
 {
-    return m->dom->nbands == 27 ? launch_cg<27>(m, cfg, mode) : launch_cg<9>(m, cfg, mode);
+    if (m->dom->nbands == 27)
+        return cfg == 0 ? launch_band_t<27, 3, 1>(m, mode, iters) : launch_band_t<27, 2, 2>(m, mode, iters);
+    return cfg == 0 ? launch_band_t<9, 3, 1>(m, mode, iters) : launch_band_t<9, 2, 2>(m, mode, iters);
 }
 
 // ---- the FP32 iteration on the element coefficients (rg_cg_coef.cuh)
@@ -1805,16 +1850,16 @@ int launch_coef_start(Matrix* m, int mode)
     return RG_OK;
 }
 
-// FP32 iterations on the element coefficients until the device flags done
-int run_coef(Matrix* m, int cfg, long long cap, long long* iters, int* status)
+// FP32 iterations with the workspace's current operator until the device flags done
+int run_f32(Matrix* m, int cfg, long long cap, long long* iters, int* status)
 {
     Workspace* w = m->ws;
     // about 20 ms of iterations per launch
-    const double iter_s = (double)m->dom->n * 60 / 5.0e12 + 3e-6;
+    const double iter_s = (double)m->dom->n * (w->coef_op ? 60 : 60 + 4 * m->dom->nbands) / 5.0e12 + 3e-6;
     const int chunk = (int)std::min(std::max(0.02 / iter_s, 16.0), 8192.0);
     long long launched = 0;
     for (;;) {
-        int rc = launch_coef(m, cfg, chunk);
+        int rc = w->coef_op ? launch_coef(m, cfg, chunk) : launch_band_cfg(m, cfg, 0, chunk);
         if (rc || (rc = read_scal(w))) return rc;
         launched += chunk;
         if (w->hs->done) break;
@@ -1885,12 +1930,7 @@ int tune_spmv(Matrix* m)
         w->hs->pk = 0;
         w->hs->norm = 1.0;
         if ((rc = write_scal_fields(w, 0.0, 1LL << 40, 0))) break;  // done = 0, no iteration cap
-        auto iterate = [&](int count) {
-            if (coef) return launch_coef(m, cfg, count);
-            int r = RG_OK;
-            for (int k = 0; k < count && r == RG_OK; ++k) r = launch_band_cfg(m, cfg);
-            return r;
-        };
+        auto iterate = [&](int count) { return coef ? launch_coef(m, cfg, count) : launch_band_cfg(m, cfg, 0, count); };
         rc = iterate(2);
         RG_CHECK_CUDA(cudaEventRecord(e0, stream()));
         if (rc == RG_OK) rc = iterate(8);
@@ -1910,13 +1950,6 @@ int tune_spmv(Matrix* m)
     slot = m->force_spmv >= 0 ? m->force_spmv : best_cfg;
     w->grid_upd32 = 0;  // the iteration has no separate update kernel
     return RG_OK;
-}
-
-int f32_step(Matrix* m)
-{
-    Workspace* w = m->ws;
-    const int cfg = cfg_slot(w);
-    return launch_band_cfg(m, cfg < 0 ? 0 : cfg, 0);
 }
 
 // balance (first solve only) and the preconditioner data (paso Solver.cpp:98,177)
@@ -2076,7 +2109,6 @@ int solve_f32(Matrix* m, const rg_solver_opts* o, OuterState& st, rg_diag& dg)
     Workspace* w = m->ws;
     const int64_t n = m->dom->n;
     const int eg = grid_for(n, kThreads, 8);
-    const int chunk = chunk_for(n, 4 * 27 + 40);  // bytes per row of a band iteration
     // segment reduction factor: 1e-2 keeps the FP32 recurrence within a few ulps of the
     // true residual (smaller factors let it drift and cost iterations)
     const double seg = std::fmin(std::fmax(o->inner_tolerance > 0 ? o->inner_tolerance : 1e-2, 1e-4), 0.5);
@@ -2109,7 +2141,7 @@ int solve_f32(Matrix* m, const rg_solver_opts* o, OuterState& st, rg_diag& dg)
         w->hs->status = ST_RUN;
         RG_CHECK_CUDA(cudaMemcpyAsync(&w->s->status, &w->hs->status, sizeof(int), cudaMemcpyHostToDevice, stream()));
         const int cfg = cfg_slot(w);
-        rc = w->coef_op ? launch_coef_start(m, first ? 1 : 2) : launch_band_cfg(m, cfg < 0 ? 0 : cfg, first ? 1 : 2);
+        rc = w->coef_op ? launch_coef_start(m, first ? 1 : 2) : launch_band_cfg(m, cfg < 0 ? 0 : cfg, first ? 1 : 2, 1);
         if (rc) return rc;
         if ((rc = read_scal(w))) return rc;
         if (w->hs->status == ST_BREAK || w->hs->status == ST_TIMEOUT) {
@@ -2125,9 +2157,7 @@ int solve_f32(Matrix* m, const rg_solver_opts* o, OuterState& st, rg_diag& dg)
         if ((rc = write_scal_fields(w, tol, cap > 0 ? cap : 1, 0))) return rc;
         long long it = 0;
         int dst = ST_RUN;
-        rc = w->coef_op ? run_coef(m, cfg < 0 ? 1 : cfg, cap, &it, &dst)
-                        : run_until_done(m, 2, f32_step, chunk, cap, &it, &dst);
-        if (rc) return rc;
+        if ((rc = run_f32(m, cfg < 0 ? 1 : cfg, cap, &it, &dst))) return rc;
         st.totIter += it;
         done_iters += it;
         if (dst == ST_TIMEOUT) {
