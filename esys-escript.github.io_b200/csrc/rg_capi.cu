@@ -375,6 +375,7 @@ int rg_matrix_values(rg_matrix* mat, double** val)
 {
     RG_REQUIRE(mat && val, "rg_matrix_values: NULL argument");
     *val = mat->m.val;
+    mat->m.values_out = true;
     return RG_OK;
 }
 

@@ -23,7 +23,8 @@ int64_t khat_size(const Domain* d) { return d->n + d->nn[0] * d->nn[1] + d->nn[0
 // Gauss points when EXPANDED; PER_ELEMENT drops q; CONSTANT also drops e); *bad = 1 where A is
 // not kappa I with the same kappa >= 0 at every point.  khat[upper corner of e] += kappa.
 __global__ void k_coef_record(int dim, int64_t ne0, int64_t ne1, int64_t nel, int64_t nn0, int64_t nn01,
-                              const double* __restrict__ A, int kind, float* __restrict__ khat, int* __restrict__ bad)
+                              const double* __restrict__ A, int kind, float* __restrict__ khat,
+                              double* __restrict__ khat64, int* __restrict__ bad)
 {
     const int dd = dim * dim;
     const int npts = kind == RG_COEF_EXPANDED ? (1 << dim) : 1;
@@ -38,14 +39,19 @@ __global__ void k_coef_record(int dim, int64_t ne0, int64_t ne1, int64_t nel, in
         const int64_t ex = e % ne0, ey = (e / ne0) % ne1, ez = e / (ne0 * ne1);
         const int64_t node = (ex + 1) + nn0 * (ey + 1) + (dim == 3 ? nn01 * (ez + 1) : 0);
         khat[node] += (float)k;
+        khat64[node] += k;
     }
 }
 
 // the nodes insertConstraint fixes (q > 0) get the sign bit of khat
-__global__ void k_coef_mask(int64_t n, const double* __restrict__ q, float* __restrict__ khat)
+__global__ void k_coef_mask(int64_t n, const double* __restrict__ q, float* __restrict__ khat,
+                            double* __restrict__ khat64)
 {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        if (q[i] > 0.0) khat[i] = -fabsf(khat[i]);
+        if (q[i] > 0.0) {
+            khat[i] = -fabsf(khat[i]);
+            khat64[i] = -fabs(khat64[i]);
+        }
 }
 
 // khat zeroed (state 0 -> the record starts)
@@ -55,7 +61,9 @@ int coef_begin(Matrix* m)
     const Domain* d = m->dom;
     if (!c.khat) RG_CHECK_CUDA(dev_malloc((void**)&c.khat, sizeof(float) * khat_size(d)));
     if (!c.bad) RG_CHECK_CUDA(dev_malloc((void**)&c.bad, sizeof(int)));
+    if (!c.khat64) RG_CHECK_CUDA(dev_malloc((void**)&c.khat64, sizeof(double) * khat_size(d)));
     RG_CHECK_CUDA(cudaMemsetAsync(c.khat, 0, sizeof(float) * khat_size(d), stream()));
+    RG_CHECK_CUDA(cudaMemsetAsync(c.khat64, 0, sizeof(double) * khat_size(d), stream()));
     RG_CHECK_CUDA(cudaMemsetAsync(c.bad, 0, sizeof(int), stream()));
     c.state = 1;
     return RG_OK;
@@ -88,7 +96,8 @@ int coef_on_assemble(Matrix* m, const rg_coef* c[6], bool reduced)
     const int64_t nel = d->ne[0] * d->ne[1] * d->ne[2];
     const int grid = grid_for(nel, 256, 8);
     k_coef_record<<<grid, 256, 0, stream()>>>(d->dim, d->ne[0], d->ne[1], nel, d->nn[0], d->nn[0] * d->nn[1],
-                                              static_cast<const double*>(c[0]->ptr), c[0]->kind, r.khat, r.bad);
+                                              static_cast<const double*>(c[0]->ptr), c[0]->kind, r.khat, r.khat64,
+                                              r.bad);
     RG_CHECK_LAUNCH();
     return RG_OK;
 }
@@ -105,7 +114,7 @@ int coef_on_constraint(Matrix* m, const double* q)
         if (rc) return rc;
     }
     const Domain* d = m->dom;
-    k_coef_mask<<<grid_for(d->n, 256, 8), 256, 0, stream()>>>(d->n, q, r.khat);
+    k_coef_mask<<<grid_for(d->n, 256, 8), 256, 0, stream()>>>(d->n, q, r.khat, r.khat64);
     RG_CHECK_LAUNCH();
     r.constrained = true;
     return RG_OK;
@@ -130,6 +139,7 @@ int coef_usable(Matrix* m, bool* usable)
 void free_coef(Matrix* m)
 {
     if (m->coef.khat) dev_free(m->coef.khat);
+    if (m->coef.khat64) dev_free(m->coef.khat64);
     if (m->coef.bad) dev_free(m->coef.bad);
     m->coef = CoefRecord();
 }

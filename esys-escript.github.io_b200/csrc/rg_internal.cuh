@@ -92,6 +92,7 @@ struct CoefRecord {
     int state = 0;              // 0: values are zero, 1: khat describes them, -1: not representable
     bool constrained = false;   // a constraint was recorded (a later assembly is not representable)
     float* khat = nullptr;
+    double* khat64 = nullptr;   // the same in FP64 (paso's FP64 PCG)
     int* bad = nullptr;         // set on the device when an element's A is not kappa I with kappa >= 0
 };
 
@@ -109,6 +110,7 @@ struct Matrix {
     float* band32 = nullptr;   // [nbands][npad] FP32 copy of the balanced matrix
     double* band64 = nullptr;  // the same layout in FP64 (paso in FP64 with RG_LAYOUT_BAND)
     int force_spmv = -1;       // FP32 SpMV configuration fixed by the caller (-1: tuned)
+    bool values_out = false;   // the caller was given the values' address and may change them unseen
     float* dinv32 = nullptr;
     Workspace* ws = nullptr;
     ResidualScratch* rs = nullptr;

@@ -2,9 +2,10 @@
 // iterations.  Included by rg_solver.cu inside namespace rg, after the solver's scalars.
 //
 // An iteration is two phases, each ended by one grid-wide sum (rg_gridmail.cuh):
-//   A  (paso: rs, x smoothing of the iteration before, sum rs^2)  p = z + beta p,  v = A p,
-//      sum p.v -> alpha
-//   B  r -= alpha v, x (paso: x2) += alpha p, z = D^-1 r, sums -> beta (paso: gamma_1/2)
+//   A  (paso: of the iteration before, x2 += alpha p, rs and x smoothing, sum rs^2)  p = z + beta p,
+//      v = A p, sum p.v -> alpha
+//   B  r -= alpha v, (textbook: x += alpha p), z = D^-1 r, sums -> beta (paso: gamma_1/2)
+// (x2 waits for the next phase A because the old p and x2 are read there anyway.)
 // p is double-buffered: in phase A every row forms the new p of its neighbours from their z and
 // old p, so that no third phase (or pass over memory) is needed for the direction.
 //
@@ -16,7 +17,7 @@
 // (rows start 27 or 9 doubles apart: odd, so no bank conflicts).  A warp whose tiles all fit
 // its ring copies them once per launch.
 //
-// What bounds it: HBM at large sizes (216 B of matrix and about 17 vector accesses of 8 B per
+// What bounds it: HBM at large sizes (216 B of matrix and about 15 vector accesses of 8 B per
 // row and iteration), the two exchanges at small ones.  Measured per iteration against one
 // kernel per step replayed from CUDA graphs: Brick 128^3 paso 134 against 215 us, Rectangle
 // 200 x 200 paso 5.9 against 20 us, 403 x 297 textbook 6.4 against 15 us.
@@ -57,6 +58,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
     if (s->done) return;
     if (threadIdx.x == 0) {
         bad = 0;
+        sc.alpha = s->alpha;
         sc.beta = s->pend ? s->beta : 0.0;
         sc.g1 = s->gamma1;
         sc.g2 = s->gamma2;
@@ -111,7 +113,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
     unsigned gen = 0;
     for (int left = a.max_iters; left > 0; --left) {
         // ---------------------------------------------------------------- phase A
-        const double beta = sc.beta, g1 = sc.g1, g2 = sc.g2;
+        const double before = sc.alpha, beta = sc.beta, g1 = sc.g1, g2 = sc.g2;
         const double* pold = par ? a.p1 : a.p0;
         double* pnew = par ? a.p0 : a.p1;
         double v[2] = {0.0, 0.0};
@@ -139,7 +141,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
             const uint32_t ph = resident ? 0u : (uint32_t)((used / S) & 1);
             const double* row_val =
                 reinterpret_cast<const double*>(ring + st * kStageBytes) + (base & 1) + (kb - base);
-            double acc = 0.0, pc = 0.0;
+            double acc = 0.0, pc = 0.0, po = 0.0;
             bool waited = false;
             if (__all_sync(0xffffffffu, inner)) {
 #pragma unroll
@@ -155,7 +157,10 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
                     for (int m = 0; m < 9; ++m) {
                         const double pn = fma(beta, pp[m], zz[m]);
                         acc = fma(row_val[3 * g + m], pn, acc);
-                        if (3 * g + m == NB / 2) pc = pn;
+                        if (3 * g + m == NB / 2) {
+                            pc = pn;
+                            po = pp[m];
+                        }
                     }
                 }
             } else {
@@ -182,7 +187,10 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
                         const double av = ok[m] ? row_val[e] : 0.0;
                         e += ok[m] ? 1 : 0;
                         if (ok[m]) acc = fma(av, pn, acc);
-                        if (3 * g + m == NB / 2) pc = pn;
+                        if (3 * g + m == NB / 2) {
+                            pc = pn;
+                            po = pp[m];
+                        }
                     }
                 }
             }
@@ -201,7 +209,9 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
                 if (PASO && pend) {
                     const double rn = g2 * rs + g1 * rr;
                     a.rs[row] = rn;
-                    a.x[row] = g2 * xx + g1 * xx2;
+                    const double xn = xx2 + before * po;
+                    a.x2[row] = xn;
+                    a.x[row] = g2 * xx + g1 * xn;
                     v[1] += rn * rn;
                 }
             }
@@ -219,10 +229,13 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
                 if (frow[h] >= 0) {
                     fr[h] = a.r[frow[h]];
                     fq[h] = a.q[frow[h]];
-                    fp[h] = pnew[frow[h]];
                     fd[h] = __ldg(a.dinv + frow[h]);
-                    fx[h] = PASO ? a.x2[frow[h]] : a.x[frow[h]];
-                    if (PASO) frs[h] = a.rs[frow[h]];
+                    if (PASO) {
+                        frs[h] = a.rs[frow[h]];
+                    } else {
+                        fp[h] = pnew[frow[h]];
+                        fx[h] = a.x[frow[h]];
+                    }
                 }
             }
         };
@@ -264,7 +277,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
                     a.r[frow[h]] = rn;
                     const double zn = rn * fd[h];
                     a.z[frow[h]] = zn;
-                    (PASO ? a.x2 : a.x)[frow[h]] = fx[h] + alpha * fp[h];
+                    if (!PASO) a.x[frow[h]] = fx[h] + alpha * fp[h];
                     u[0] += zn * rn;
                     if (PASO) {
                         const double d = rn - frs[h];

@@ -71,6 +71,8 @@ struct Workspace {
     double *r = nullptr, *x = nullptr, *rs = nullptr, *x2 = nullptr, *q = nullptr, *z = nullptr;
     double* p = nullptr;
     double* p2 = nullptr;  // the persistent FP64 PCG's second buffer of p
+    double* bvm = nullptr; // its signed balance vector when the operator is marched
+    bool coef64 = false;   // the current FP64 solve marches the operator from the coefficients
     unsigned long long* mail = nullptr;  // its grid-wide sums (rg_gridmail.cuh)
     double* bb = nullptr;  // balanced rhs
     float* d32 = nullptr;                // FP32 path: correction accumulated over a segment
@@ -1142,6 +1144,8 @@ __global__ void __launch_bounds__(kTile + 32, kCtas) k_f32_cg(const float* __res
 
 #include "rg_cg_coef.cuh"
 
+#include "rg_pcg64_coef.cuh"
+
 // The element-coefficient operator's seed: the balanced FP64 residual is unbalanced (r =
 // r64 / bv, scaled by inv_scale); fixed nodes get their exact correction d = r (identity
 // rows) and a zero state; free rows u = r / diag (z, p, d = 0 when fresh).
@@ -1452,6 +1456,7 @@ TmaBandArgs band_offsets(const Domain* d)
 }
 
 int sm_count();
+void q1_table(const Domain* d, double (&T)[8]);
 
 // FP64 band kernel (SpMV or Jacobi sweep) over all tiles, one CTA per SM.  The vector x that
 // is bulk-copied is always a solver workspace array (cudaMalloc: 256-byte aligned).  Launch
@@ -1595,6 +1600,71 @@ int run_pcg64_t(Matrix* m, long long cap, long long* iters, int* status)
             return RG_TIMEOUT;
         }
     }
+    *iters = w->hs->iter;
+    *status = w->hs->status;
+    return RG_OK;
+}
+
+// paso's FP64 PCG on the element coefficients, from k_paso_init's state until the device flags done
+constexpr int kCoef64Warps = 16;
+// rows of a 3D grid from which the marched operator is used.  Against the CSR values (whole solve): 48 x 50
+// x 52 (137,000 rows) 3.93 against 3.77 ms, 64^3 (275,000) 6.71 against 8.56, 80 x 70 x 90 11.7 against
+// 19.1, 128^3 75.9 against 116.9.  In 2D a row has 72 bytes of matrix and three planes of halo to march:
+// 500 x 420 29.6 against 22.4 ms, 1000 x 1200 269 against 246.
+constexpr int64_t kCoef64Rows = 200000;
+
+int run_pcg64_coef(Matrix* m, long long cap, long long* iters, int* status)
+{
+    constexpr int DIM = 3, W = kCoef64Warps;
+    Workspace* w = m->ws;
+    const Domain* d = m->dom;
+    const int64_t n = d->n;
+    if (!w->p2) RG_CHECK_CUDA(dev_malloc((void**)&w->p2, sizeof(double) * n));
+    if (!w->bvm) RG_CHECK_CUDA(dev_malloc((void**)&w->bvm, sizeof(double) * n));
+    const int eg = grid_for(n, kThreads, 8);
+    RG_TIMED(T_VECTOR, (k_pcg64_coef_enter<<<eg, kThreads, 0, stream()>>>(n, m->coef.khat64, m->bv, w->bvm, w->z, w->p,
+                                                                          w->x, w->x2)));
+    RG_CHECK_LAUNCH();
+    Pcg64CoefArgs a{};
+    double T[8];
+    q1_table(d, T);
+    a.t = march_table<double>(d->dim, T);
+    const int ctas = std::min(sm_count(), kMailCtas);
+    a.g = march_geom(d->dim, d->nn, 1, ctas, W);
+    a.khat = m->coef.khat64;
+    a.r = w->r;
+    a.q = w->q;
+    a.rs = w->rs;
+    a.x = w->x;
+    a.x2 = w->x2;
+    a.z = w->z;
+    a.p0 = w->p;
+    a.p1 = w->p2;
+    a.dinv = m->dinv;
+    a.bvm = w->bvm;
+    a.mail = w->mail;
+    const double iter_s = (double)n * 180 / 5.0e12 + 6e-6;  // about 20 ms of iterations per launch
+    a.max_iters = (int)std::min(std::max(0.02 / iter_s, 16.0), 8192.0);
+    const int grid = march_ctas(a.g, ctas);
+    long long launched = 0;
+    for (;;) {
+        RG_CHECK_CUDA(cudaMemsetAsync(w->mail, 0, kMailBytes, stream()));
+        void* args[] = {&a, &w->s};
+        cudaError_t e;
+        RG_TIMED(T_PASO_SPMV, (e = cudaLaunchCooperativeKernel((const void*)k_pcg64_coef<DIM, W>, dim3(grid), dim3(W * 32),
+                                                               args, 0, stream())));
+        RG_CHECK_CUDA(e);
+        launched += a.max_iters;
+        int rc = read_scal(w);
+        if (rc) return rc;
+        if (w->hs->done) break;
+        if (launched > cap + 2LL * a.max_iters + 8) {
+            set_error("PCG iteration loop did not terminate");
+            return RG_TIMEOUT;
+        }
+    }
+    RG_TIMED(T_VECTOR, (k_pcg64_coef_leave<<<eg, kThreads, 0, stream()>>>(n, m->bv, w->x)));
+    RG_CHECK_LAUNCH();
     *iters = w->hs->iter;
     *status = w->hs->status;
     return RG_OK;
@@ -2088,6 +2158,7 @@ int solve_fp64(Matrix* m, const rg_solver_opts* o, bool paso, OuterState& st, rg
             RG_CHECK_LAUNCH();
             // more than one Jacobi sweep has an SpMV inside the preconditioner: one kernel per step
             rc = w->sweeps > 1 ? run_until_done(m, 0, paso_step, chunk, cnt, &it, &dst)
+                 : w->coef64   ? run_pcg64_coef(m, cnt, &it, &dst)
                                : run_pcg64(m, true, cnt, &it, &dst);
             if (rc) return rc;
         } else {
@@ -2279,7 +2350,7 @@ void free_workspace(Matrix* m)
 {
     Workspace* w = m->ws;
     if (!w) return;
-    double* dd[] = {w->r, w->x, w->rs, w->x2, w->q, w->z, w->p, w->p2, w->bb, w->partials};
+    double* dd[] = {w->r, w->x, w->rs, w->x2, w->q, w->z, w->p, w->p2, w->bvm, w->bb, w->partials};
     for (double* p : dd) dev_free(p);
     dev_free(w->mail);
     dev_free(w->d32);
@@ -2382,6 +2453,9 @@ int solve_impl(Matrix* m, const double* rhs, double* x, const rg_solver_opts* o,
     bool coef = false;
     if (fp32 && o->layout == RG_LAYOUT_COEF && (rc = coef_usable(m, &coef))) return rc;
     if ((rc = prepare(m, fp32 && !coef, band64))) return rc;
+    bool coef64 = false;
+    if (paso && o->sweeps <= 1 && d->dim == 3 && n >= kCoef64Rows && !m->values_out && (rc = coef_usable(m, &coef64))) return rc;
+    w->coef64 = coef64;
     w->band64 = band64;
     w->coef_op = coef;
     dg.inner_operator = coef ? 1 : 0;

@@ -756,6 +756,7 @@ __global__ void __launch_bounds__(kSysWarps * 32, 1) k_pcg_sys(const __grid_cons
     if (s->done) return;
     if (threadIdx.x == 0) {
         bad = 0;
+        sc.alpha = s->alpha;
         sc.beta = s->pend ? s->beta : 0.0;
         sc.g1 = s->gamma1;
         sc.g2 = s->gamma2;
@@ -808,7 +809,7 @@ __global__ void __launch_bounds__(kSysWarps * 32, 1) k_pcg_sys(const __grid_cons
     unsigned gen = 0;
     for (int left = a.max_iters; left > 0; --left) {
         // ---------------------------------------------------------------- phase A
-        const double beta = sc.beta, g1 = sc.g1, g2 = sc.g2;
+        const double before = sc.alpha, beta = sc.beta, g1 = sc.g1, g2 = sc.g2;
         const double* pold = par ? a.p1 : a.p0;
         double* pnew = par ? a.p0 : a.p1;
         double v[2] = {0.0, 0.0};
@@ -892,7 +893,9 @@ __global__ void __launch_bounds__(kSysWarps * 32, 1) k_pcg_sys(const __grid_cons
                 if (pend) {
                     const double rn = g2 * rs + g1 * rr;
                     a.rs[o] = rn;
-                    a.x[o] = g2 * xx + g1 * xx2;
+                    const double xn = xx2 + before * po;
+                    a.x2[o] = xn;
+                    a.x[o] = g2 * xx + g1 * xn;
                     v[1] += rn * rn;
                 }
             }
@@ -921,14 +924,12 @@ __global__ void __launch_bounds__(kSysWarps * 32, 1) k_pcg_sys(const __grid_cons
             const int node = (tb + run * tstep) * kTileNodes + (i - run * per_run);
             if (node >= a.n) continue;
             const int64_t o = (int64_t)node * NB;
-            double rn[NB], qq[NB], rs[NB], xx[NB], pp[NB], di[B2];
+            double rn[NB], qq[NB], rs[NB], di[B2];
 #pragma unroll
             for (int c = 0; c < NB; ++c) {
                 rn[c] = a.r[o + c];
                 qq[c] = a.q[o + c];
                 rs[c] = a.rs[o + c];
-                xx[c] = a.x2[o + c];
-                pp[c] = pnew[o + c];
             }
 #pragma unroll
             for (int c = 0; c < B2; ++c) di[c] = __ldg(a.dinv + (int64_t)node * B2 + c);
@@ -939,7 +940,6 @@ __global__ void __launch_bounds__(kSysWarps * 32, 1) k_pcg_sys(const __grid_cons
                 const double d = rn[c] - rs[c];
                 u[1] += d * d;
                 u[2] += d * rs[c];
-                a.x2[o + c] = xx[c] + alpha * pp[c];
             }
 #pragma unroll
             for (int e = 0; e < NB; ++e) {

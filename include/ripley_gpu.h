@@ -95,7 +95,9 @@ int rg_matrix_create_system(rg_domain* dom, int block_size, rg_matrix** out);
 int rg_matrix_block_size(const rg_matrix* mat, int* block_size);
 /* AbstractSystemMatrix::resetValues: zero the values, drop balancing and solver data */
 int rg_matrix_reset(rg_matrix* mat);
-/* device pointer to the nnz CSR values (FP64), in the domain's pattern order */
+/* device pointer to the nnz CSR values (FP64), in the domain's pattern order.  FP64 solves of a matrix
+   whose values were handed out read them; otherwise paso's PCG on a large 3D grid may evaluate the same
+   operator from the element coefficients it was assembled from. */
 int rg_matrix_values(rg_matrix* mat, double** val);
 /* 1 when the values have been balanced in place by a solve (paso keeps them so) */
 int rg_matrix_is_balanced(const rg_matrix* mat, int* balanced);
