@@ -6,9 +6,15 @@
 // not).  Device blocks therefore come from a stream-ordered pool of the library's own, one per device,
 // which keeps at most kKept bytes that nothing uses and returns what is above it to the device at the next
 // synchronisation; pinned blocks of 1 KiB are kept in a list of at most kPinned.  Both are safe for
-// several threads.  As with cudaFree, a block is given back only when the device has finished all work:
+// several threads.  Large blocks (kDirect) and blocks asked for while the caller's stream is being captured
+// (which cudaMalloc refuses or allows by the capture's mode, where the pool would hand out a block of the
+// graph) come from cudaMalloc: kernels
+// on arrays of hundreds of MB run slower on the pool's memory (a batch of 12 Bricks x 8 right hand sides 344
+// against 322 ms) and growing the pool by gigabytes takes longer than cudaMalloc (creating a 256^3 grid and
+// matrix 70 to 90 against 6 to 11 ms).  As with cudaFree, a block is given back only when the device has finished all work:
 // the caller may still use it on a stream that the library does not know.
 #include <mutex>
+#include <unordered_set>
 #include <vector>
 
 #include "rg_internal.cuh"
@@ -17,6 +23,7 @@ namespace rg {
 namespace {
 
 constexpr uint64_t kKept = 2ull << 30;
+constexpr size_t kDirect = 64ull << 20;
 constexpr size_t kPinned = 32;
 constexpr int kMaxDevices = 64;
 
@@ -54,6 +61,23 @@ cudaMemPool_t pool()
     return pools[dev];
 }
 
+// the blocks that came from cudaMalloc although there is a pool
+std::unordered_set<void*>& direct()
+{
+    static std::unordered_set<void*> set;
+    return set;
+}
+
+bool capturing()
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream(), &st) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return st != cudaStreamCaptureStatusNone;
+}
+
 std::vector<void*>& pinned()
 {
     static std::vector<void*> list;
@@ -67,6 +91,19 @@ cudaError_t dev_malloc(void** p, size_t bytes)
     *p = nullptr;
     cudaMemPool_t mp = pool();
     if (!mp) return cudaMalloc(p, bytes ? bytes : 1);
+    if (bytes >= kDirect || capturing()) {
+        cudaError_t e = cudaMalloc(p, bytes ? bytes : 1);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            cudaMemPoolTrimTo(mp, 0);
+            e = cudaMalloc(p, bytes ? bytes : 1);
+        }
+        if (e == cudaSuccess) {
+            std::lock_guard<std::mutex> lock(mutex());
+            direct().insert(*p);
+        }
+        return e;
+    }
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes ? bytes : 1, mp, stream());
     if (e == cudaErrorMemoryAllocation) {
         // what the pool keeps unused may be what is missing
@@ -88,7 +125,12 @@ void dev_free(void* p)
         return;
     }
     if (at.device != dev) cudaSetDevice(at.device);
-    if (pool()) {
+    bool own = true;
+    {
+        std::lock_guard<std::mutex> lock(mutex());
+        own = direct().erase(p) == 0;
+    }
+    if (own && pool()) {
         cudaDeviceSynchronize();
         cudaFreeAsync(p, nullptr);
     } else {
