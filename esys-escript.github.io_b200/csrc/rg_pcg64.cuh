@@ -19,7 +19,7 @@
 //
 // What bounds it: HBM at large sizes (216 B of matrix and about 15 vector accesses of 8 B per
 // row and iteration), the two exchanges at small ones.  Measured per iteration against one
-// kernel per step replayed from CUDA graphs: Brick 128^3 paso 134 against 215 us, Rectangle
+// kernel per step replayed from CUDA graphs: Brick 128^3 paso 130 against 215 us, Rectangle
 // 200 x 200 paso 5.9 against 20 us, 403 x 297 textbook 6.4 against 15 us.
 #pragma once
 
@@ -164,29 +164,32 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
                     }
                 }
             } else {
-                waited = mbar_wait(&full[warp][st], ph, polls);
+                // a tile with boundary rows (half of them at lines of 129 nodes): the same nine loads at a time,
+                // a missing neighbour's from the row itself; its entry is left out.  ok9: which of the 3 x 3
+                // neighbours (x, y) of a plane exist.  Loaded three at a time after the wait, solves took: 95 x
+                // 97 x 96 paso 37.0 ms (now 32.3), textbook 41.8 (30.7); 128^3 100.7 (96.8) and 98.7 (94.5).
                 const int rowc = in ? row : row0;
+                const unsigned x3 = !in ? 0u : (cx > 0 ? 1u : 0u) | 2u | (cx + 1 < (unsigned)a.nn0 ? 4u : 0u);
+                const unsigned ok9 = (cy > 0 ? x3 : 0u) | x3 << 3 | (cy + 1 < (unsigned)a.nn1 ? x3 << 6 : 0u);
                 int e = 0;
 #pragma unroll
-                for (int g = 0; g < NB / 3; ++g) {
-                    const int dy = g % 3, dz = g / 3;
-                    const bool gv = in && (dy == 0 ? cy > 0 : (dy == 2 ? cy + 1 < (unsigned)a.nn1 : true)) &&
-                                    (NB == 9 || (dz == 0 ? cz > 0 : (dz == 2 ? cz + 1 < (unsigned)a.nn2 : true)));
-                    double zz[3], pp[3];
-                    bool ok[3];
+                for (int g = 0; g < NB / 3; g += 3) {
+                    const bool zv = NB == 9 || (g == 0 ? cz > 0 : (g == 6 ? cz + 1 < (unsigned)a.nn2 : true));
+                    const unsigned okg = zv ? ok9 : 0u;
+                    double zz[9], pp[9];
 #pragma unroll
-                    for (int m = 0; m < 3; ++m) {
-                        ok[m] = gv && (m == 0 ? cx > 0 : (m == 2 ? cx + 1 < (unsigned)a.nn0 : true));
-                        const int j = ok[m] ? row + a.off[3 * g + m] : rowc;
+                    for (int m = 0; m < 9; ++m) {
+                        const int j = okg >> m & 1u ? row + a.off[3 * g + m] : rowc;
                         zz[m] = a.z[j];
                         pp[m] = pold[j];
                     }
+                    if (g == 0) waited = mbar_wait(&full[warp][st], ph, polls);
 #pragma unroll
-                    for (int m = 0; m < 3; ++m) {
+                    for (int m = 0; m < 9; ++m) {
                         const double pn = fma(beta, pp[m], zz[m]);
-                        const double av = ok[m] ? row_val[e] : 0.0;
-                        e += ok[m] ? 1 : 0;
-                        if (ok[m]) acc = fma(av, pn, acc);
+                        const bool ok = okg >> m & 1u;
+                        if (ok) acc = fma(row_val[e], pn, acc);
+                        e += ok ? 1 : 0;
                         if (3 * g + m == NB / 2) {
                             pc = pn;
                             po = pp[m];
