@@ -3,9 +3,10 @@
 //
 // An iteration is two phases, each ended by one grid-wide sum (rg_gridmail.cuh):
 //   A  (paso: of the iteration before, x2 += alpha p, rs and x smoothing, sum rs^2)  p = z + beta p,
-//      v = A p, sum p.v -> alpha
-//   B  r -= alpha v, (textbook: x += alpha p), z = D^-1 r, sums -> beta (paso: gamma_1/2)
-// (x2 waits for the next phase A because the old p and x2 are read there anyway.)
+//      v = A p, sum p.v -> alpha; textbook: x += alpha p of the iteration before
+//   B  r -= alpha v, z = D^-1 r, sums -> beta (paso: gamma_1/2)
+// (x2, and the textbook x, wait for the next phase A because the old p is read there anyway; the textbook
+// x takes its last step when the launch ends.)
 // p is double-buffered: in phase A every row forms the new p of its neighbours from their z and
 // old p, so that no third phase (or pass over memory) is needed for the direction.
 //
@@ -110,6 +111,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
             for (int k = 0; k < (resident ? mine : S); ++k) issue();
     }
 
+    bool xpend = false;           // textbook: whether x has yet to take alpha p
     unsigned gen = 0;
     for (int left = a.max_iters; left > 0; --left) {
         // ---------------------------------------------------------------- phase A
@@ -128,6 +130,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
                 xx = a.x[row];
                 xx2 = a.x2[row];
             }
+            if (!PASO && xpend && in) xx = a.x[row];
             const int kb = __ldg(a.ptr + (in ? row : row0));
             const int base = __shfl_sync(0xffffffffu, kb, 0);
             const unsigned plane = a.nn0 * a.nn1;
@@ -209,6 +212,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
                 pnew[row] = pc;
                 a.q[row] = acc;
                 v[0] += acc * pc;
+                if (!PASO && xpend) a.x[row] = xx + before * po;
                 if (PASO && pend) {
                     const double rn = g2 * rs + g1 * rr;
                     a.rs[row] = rn;
@@ -222,7 +226,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
         // phase B walks the tiles backwards (the rows phase A touched last are the likeliest in L2),
         // two per step; a thread's rows are those it had in phase A, so all it reads but alpha is its
         // own work: the first pair is loaded before the exchange, whose wait covers the loads
-        double fr[2], fq[2], frs[2], fx[2], fp[2], fd[2];
+        double fr[2], fq[2], frs[2], fd[2];
         int frow[2];
         auto fetch = [&](int k) {
 #pragma unroll
@@ -233,12 +237,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
                     fr[h] = a.r[frow[h]];
                     fq[h] = a.q[frow[h]];
                     fd[h] = __ldg(a.dinv + frow[h]);
-                    if (PASO) {
-                        frs[h] = a.rs[frow[h]];
-                    } else {
-                        fp[h] = pnew[frow[h]];
-                        fx[h] = a.x[frow[h]];
-                    }
+                    if (PASO) frs[h] = a.rs[frow[h]];
                 }
             }
         };
@@ -266,6 +265,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
         }
         __syncthreads();
         par ^= 1;
+        xpend = false;
         if (sc.stop) break;
 
         // ---------------------------------------------------------------- phase B
@@ -280,7 +280,6 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
                     a.r[frow[h]] = rn;
                     const double zn = rn * fd[h];
                     a.z[frow[h]] = zn;
-                    if (!PASO) a.x[frow[h]] = fx[h] + alpha * fp[h];
                     u[0] += zn * rn;
                     if (PASO) {
                         const double d = rn - frs[h];
@@ -317,7 +316,16 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
         }
         __syncthreads();
         pend = true;
+        xpend = !PASO;
         if (sc.stop) break;
+    }
+    if (!PASO && xpend) {
+        const double alpha = sc.alpha;
+        const double* p = par ? a.p1 : a.p0;
+        for (int k = 0; k < mine; ++k) {
+            const int row = (t0 + k * tstep) * 32 + lane;
+            if (row < a.n) a.x[row] = a.x[row] + alpha * p[row];
+        }
     }
     // copies still in flight land (bounded) before the ring is given up
     if (lane == 0) {

@@ -6,13 +6,14 @@
 // not).  Device blocks therefore come from a stream-ordered pool of the library's own, one per device,
 // which keeps at most kKept bytes that nothing uses and returns what is above it to the device at the next
 // synchronisation; pinned blocks of 1 KiB are kept in a list of at most kPinned.  Both are safe for
-// several threads.  Large blocks (kDirect) and blocks asked for while the caller's stream is being captured
-// (which cudaMalloc refuses or allows by the capture's mode, where the pool would hand out a block of the
-// graph) come from cudaMalloc: kernels
-// on arrays of hundreds of MB run slower on the pool's memory (a batch of 12 Bricks x 8 right hand sides 344
-// against 322 ms) and growing the pool by gigabytes takes longer than cudaMalloc (creating a 256^3 grid and
-// matrix 70 to 90 against 6 to 11 ms).  As with cudaFree, a block is given back only when the device has finished all work:
+// several threads.  As with cudaFree, a block is given back only when the device has finished all work:
 // the caller may still use it on a stream that the library does not know.
+//
+// Large blocks (kDirect) come from cudaMalloc: kernels on arrays of hundreds of MB run slower on the pool's
+// memory (a batch of 12 Bricks x 8 right hand sides 344 against 322 ms), and growing the pool by gigabytes
+// takes longer (creating a 256^3 grid and matrix 70 to 90 against 6 to 11 ms).  So do blocks asked for while
+// the caller's stream is captured, which cudaMalloc refuses or allows by the capture's mode; the pool would
+// hand out a block of the graph.
 #include <mutex>
 #include <unordered_set>
 #include <vector>
