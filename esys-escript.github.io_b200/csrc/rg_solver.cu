@@ -551,6 +551,73 @@ __global__ void __launch_bounds__(kThreads) k_std_init(int64_t n, const double* 
     }
 }
 
+// x += alpha p; r -= alpha q; z = dinv r; rho_next = r.z, ||r||^2; stopping tests; beta
+__global__ void __launch_bounds__(kThreads) k_std_update(int64_t n, double* __restrict__ x,
+                                                         double* __restrict__ r,
+                                                         const double* __restrict__ q,
+                                                         const double* __restrict__ p,
+                                                         const double* __restrict__ dinv,
+                                                         double* __restrict__ z, ReduceBuf rb, Scal* s)
+{
+    if (s->done) return;
+    const double alpha = s->alpha;
+    double v[2] = {0.0, 0.0};
+    const int64_t nv = n >> 1;
+    for (int64_t k = gtid(); k < nv; k += gstride()) {
+        const double2 x0 = ld2(x, k), r0 = ld2(r, k), q0 = ld2(q, k), p0 = ld2(p, k), di = ld2(dinv, k);
+        st2(x, k, make_double2(x0.x + alpha * p0.x, x0.y + alpha * p0.y));
+        const double ra = r0.x - alpha * q0.x, rb2 = r0.y - alpha * q0.y;
+        st2(r, k, make_double2(ra, rb2));
+        const double za = ra * di.x, zb = rb2 * di.y;
+        st2(z, k, make_double2(za, zb));
+        v[0] += za * ra + zb * rb2;
+        v[1] += ra * ra + rb2 * rb2;
+    }
+    if ((n & 1) && gtid() == 0) {
+        const int64_t i = n - 1;
+        x[i] += alpha * p[i];
+        const double ri = r[i] - alpha * q[i];
+        r[i] = ri;
+        const double zi = ri * dinv[i];
+        z[i] = zi;
+        v[0] += zi * ri;
+        v[1] += ri * ri;
+    }
+    double t[2];
+    if (grid_reduce<2>(v, rb, t) && threadIdx.x == 0) {
+        const long long it = s->iter + 1;
+        s->iter = it;
+        const double norm = sqrt(t[1]);
+        s->norm = norm;
+        s->beta = t[0] / s->rho;
+        const bool brk = !(fabs(t[0]) > 0.0);
+        s->rho = t[0];
+        if (norm <= s->tol) {
+            s->status = ST_CONV;
+            s->done = 1;
+        } else if (it >= s->maxit) {
+            s->status = ST_MAXIT;
+            s->done = 1;
+        } else if (brk) {
+            s->status = ST_BREAK;
+            s->done = 1;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) k_std_pupdate(int64_t n, const double* __restrict__ z,
+                                                          double* __restrict__ p, const Scal* s)
+{
+    if (s->done) return;
+    const double beta = s->beta;
+    const int64_t nv = n >> 1;
+    for (int64_t k = gtid(); k < nv; k += gstride()) {
+        const double2 z0 = ld2(z, k), p0 = ld2(p, k);
+        st2(p, k, make_double2(z0.x + beta * p0.x, z0.y + beta * p0.y));
+    }
+    if ((n & 1) && gtid() == 0) p[n - 1] = z[n - 1] + beta * p[n - 1];
+}
+
 // ------------------------------------------------------------------ FP32 PCG on the band copy
 // Tile-major band layout: rows are grouped in tiles of kTile; tile T's coefficients are
 // band[(T*NB + b)*kTile + t] for row T*kTile + t and band b (neighbour i + off_b; 0 where
@@ -612,14 +679,14 @@ __global__ void __launch_bounds__(kThreads) k_cheb_step_band(const __grid_consta
     }
 }
 
-// The FP64 band kernels of the paso PCG with extra sweeps (RG_LAYOUT_BAND), warp-specialised and persistent
-// like k_f32_cg: lane 0 of warp kConsumerWarps streams, per tile, the tile's FP64 band
+// The FP64 band kernels (RG_LAYOUT_BAND: paso's PCG with extra sweeps, the textbook PCG on large 3D grids),
+// warp-specialised and persistent like k_f32_cg: lane 0 of warp kConsumerWarps streams, per tile, the tile's FP64 band
 // block (one bulk copy, L2 evict-first) and, for interior tiles, the NG windows of x its
 // stencil columns span (kTile+4 values from a 16-byte aligned start) into a kStages ring;
 // consumer warps compute row i0 + t from shared memory.  Tiles near the two ends read x with
 // clamped loads.  The bands are summed in column order.
 //   SWEEP = false: v = A x, delta = x.v, alpha = tau/delta, breakdown on delta == 0
-//                  (PCG.cpp:223-262), i.e. k_paso_spmv.
+//                  (PCG.cpp:223-262), i.e. k_paso_spmv; mode 1: alpha = rho/delta, the textbook PCG's.
 //   SWEEP = true:  one Jacobi sweep out = x + dinv (b - A x) with k_jacobi_sweep's modes.
 // All waits are bounded: on timeout the kernel records ST_TIMEOUT and returns.
 constexpr int kWin64 = kTile + 4;
@@ -755,10 +822,17 @@ __global__ void __launch_bounds__(kTile + 32, 1) k_band64_bulk(const double* __r
     if (SWEEP && mode == 0) return;
     double tt[1];
     if (grid_reduce<1>(v, rb, tt) && threadIdx.x == 0) {
-        if (!SWEEP) {
+        if (!SWEEP && mode == 0) {
             s->delta = tt[0];
             s->alpha = s->tau / tt[0];
             if (fabs(tt[0]) <= 0.0) {  // breakFlag
+                s->iter += 1;
+                report_status(s, ST_BREAK);
+            }
+        } else if (!SWEEP) {
+            s->delta = tt[0];
+            s->alpha = s->rho / tt[0];
+            if (!(fabs(tt[0]) > 0.0)) {
                 s->iter += 1;
                 report_status(s, ST_BREAK);
             }
@@ -1520,6 +1594,18 @@ int paso_step(Matrix* m)
     return RG_OK;
 }
 
+int std_band_step(Matrix* m)
+{
+    Workspace* w = m->ws;
+    const int64_t n = m->dom->n;
+    launch_band64<false>(m, w->p, w->q, nullptr, nullptr, 1);
+    RG_TIMED(T_STD_UPDATE, (k_std_update<<<w->grid_vec, kThreads, 0, stream()>>>(n, w->x, w->r, w->q, w->p, m->dinv, w->z,
+                                                                                 rbuf(w), w->s)));
+    RG_TIMED(T_VECTOR, (k_std_pupdate<<<w->grid_vec, kThreads, 0, stream()>>>(n, w->z, w->p, w->s)));
+    RG_CHECK_LAUNCH();
+    return RG_OK;
+}
+
 int sm_count()
 {
     static int count = 0;
@@ -1612,6 +1698,10 @@ constexpr int kCoef64Warps = 16;
 // 19.1, 128^3 75.9 against 116.9.  In 2D a row has 72 bytes of matrix and three planes of halo to march:
 // 500 x 420 29.6 against 22.4 ms, 1000 x 1200 269 against 246.
 constexpr int64_t kCoef64Rows = 200000;
+
+// rows of a 3D grid from which RG_LAYOUT_BAND's textbook PCG runs on the band copy, a kernel per step (whole
+// solve, against k_pcg64): 96^3 (912,673 rows) 33.0 against 30.4 ms, 128^3 (2.15 million) 87.6 against 90.3
+constexpr int64_t kBand64Rows = 1500000;
 
 int run_pcg64_coef(Matrix* m, long long cap, long long* iters, int* status)
 {
@@ -2165,7 +2255,9 @@ int solve_fp64(Matrix* m, const rg_solver_opts* o, bool paso, OuterState& st, rg
             RG_TIMED(T_VECTOR, (k_std_init<<<w->grid_rows, kThreads, 0, stream()>>>(
                                    n, w->r, m->dinv, w->z, w->p, rbuf(w), w->s, tol, cnt > 0 ? cnt : 1)));
             RG_CHECK_LAUNCH();
-            if ((rc = run_pcg64(m, false, cnt, &it, &dst))) return rc;
+            rc = w->band64 ? run_until_done(m, 1, std_band_step, chunk, cnt, &it, &dst)
+                           : run_pcg64(m, false, cnt, &it, &dst);
+            if (rc) return rc;
         }
         st.totIter += it;
         bool restart = false;
@@ -2440,9 +2532,11 @@ int solve_impl(Matrix* m, const double* rhs, double* x, const rg_solver_opts* o,
     // every grid reduction leaves the counter at zero; clearing it here as well keeps one
     // solve independent of anything an earlier, interrupted one left behind
     RG_CHECK_CUDA(cudaMemsetAsync(w->counter, 0, sizeof(unsigned), stream()));
-    // the FP64 band copy serves the extra Jacobi sweeps; with one sweep the persistent PCG streams
-    // the CSR values without their column indices, the same bytes
-    const bool band64 = paso && o->sweeps > 1 && o->layout == RG_LAYOUT_BAND;
+    // the FP64 band copy serves the extra Jacobi sweeps, and the textbook PCG where its bulk-copied tiles
+    // outweigh the launches (kBand64Rows); else one sweep streams the CSR values without their column
+    // indices, the same bytes
+    const bool band64 = !fp32 && o->layout == RG_LAYOUT_BAND &&
+                        (paso ? o->sweeps > 1 : m->dom->dim == 3 && m->dom->n >= kBand64Rows);
     if (!fp32 && o->layout == RG_LAYOUT_COEF) {
         set_error("solver: RG_LAYOUT_COEF evaluates the FP32 inner operator; FP64 solves use RG_LAYOUT_CSR or "
                   "RG_LAYOUT_BAND");
