@@ -185,12 +185,13 @@ def cpu_reference_warmup(inp, threads):
 # our arm
 # ----------------------------------------------------------------------------------------------
 
-# algorithmic bytes per launch of the dominant kernel, per DOF (n): one fused FP32 PCG
-# iteration reads the row's operator data and its 16-byte iteration state {u, D^-1 A u,
-# D^-1 A p, p}, writes the new state, and updates the correction d (read + write).  Operator
-# data: the element coefficient of the row's node (4 B, RG_LAYOUT_COEF, the timed path), or
-# the row's 27 band values (4 B each, padded bands count, RG_LAYOUT_BAND)
-F32_COEF_BYTES_PER_ROW = 4 + 16 + 16 + 8
+# algorithmic bytes per iteration of the dominant kernel, per DOF (n); a launch runs many
+# iterations.  One FP32 PCG iteration reads the row's operator data and its 16-byte iteration
+# state {u, D^-1 A u, D^-1 A p, p}, writes the new state, and updates the correction d (read +
+# write: every iteration on the band copy, every second one on the element coefficients).
+# Operator data: the element coefficient of the row's node (4 B, RG_LAYOUT_COEF, the timed
+# path), or the row's 27 band values (4 B each, padded bands count, RG_LAYOUT_BAND)
+F32_COEF_BYTES_PER_ROW = 4 + 16 + 16 + 4
 F32_SPMV_BYTES_PER_ROW = 27 * 4 + 16 + 16 + 8
 
 
@@ -347,17 +348,17 @@ def run_ours(args):
             d = step(timed)
         e1.record(stream)
         torch.cuda.synchronize()
-        # the iteration kernel's average launch time (events around every launch, one step)
+        # the iteration kernel's time per iteration (events around every launch, one step)
         lib.rg_timers_reset()
         lib.rg_timers_enable(1)
-        step(timed)
+        d = step(timed)
         torch.cuda.synchronize()
         lib.rg_timers_enable(0)
-        _, kt, kms = L.timers()["f32_spmv"]
+        kms = L.timers()["f32_spmv"][2]
         print(json.dumps({"only": "fast", "path": args.path, "iterations": int(d.num_iter),
                           "outer_steps": int(d.num_outer), "inner_operator": int(d.inner_operator),
                           "fp64_fallback": int(d.fp64_fallback), "ms_per_step": e0.elapsed_time(e1) / args.steps,
-                          "iteration_kernel_us": kms / max(kt, 1) * 1e3}), flush=True)
+                          "iteration_kernel_us": kms / max(int(d.num_iter), 1) * 1e3}), flush=True)
         return
 
     # --- FP64 reference solution for the error statement (paso algorithm, rtol 1e-10, or
@@ -432,14 +433,13 @@ def run_ours(args):
     torch.cuda.synchronize()
     f32_band_ms = max_over_ranks(ev0.elapsed_time(ev1) / n_f)
     x_f32_band = x.clone()
-    # its iteration kernel's average launch time (events around every launch, one step)
+    # its iteration kernel's time per iteration (events around every launch, one step)
     lib.rg_timers_reset()
     lib.rg_timers_enable(1)
-    step(fast_band)
+    d_fb = step(fast_band)
     torch.cuda.synchronize()
     lib.rg_timers_enable(0)
-    _, bt, bms = L.timers()["f32_spmv"]
-    band_us = bms / max(bt, 1) * 1e3
+    band_us = L.timers()["f32_spmv"][2] / max(int(d_fb.num_iter), 1) * 1e3
 
     # --- the same with A given expanded (its 9 values repeated at the 8 Gauss points, the form
     # escript's general assembler reads): the assembly reads 1.2 GB of A instead of 151 MB
@@ -471,7 +471,7 @@ def run_ours(args):
         step(timed)
     barrier()
 
-    # --- timed region: K steps of the fast path (iteration chunks replayed as CUDA graphs)
+    # --- timed region: K steps of the fast path
     gpu_id = None
     try:
         gpu_id = "GPU-" + str(torch.cuda.get_device_properties(local).uuid)
@@ -493,23 +493,25 @@ def run_ours(args):
     err = float((x_fast - x_fp64).norm() / x_fp64.norm())
 
     # --- kernel timing: the same steps with CUDA events around every library launch (on the
-    # launching stream); graphs are off while events are recorded
+    # launching stream)
     n_prof = max(1, min(args.steps, 3))
     lib.rg_timers_reset()
     lib.rg_timers_enable(1)
     barrier()
     ev0.record(stream)
+    prof_iters = 0
     for _ in range(n_prof):
-        step(timed)
+        prof_iters += int(step(timed).num_iter)
     ev1.record(stream)
     torch.cuda.synchronize()
     lib.rg_timers_enable(0)
     ms_events = ev0.elapsed_time(ev1) / n_prof
     tm = L.timers()
 
-    # dominant kernel: the fused FP32 iteration; average launch time from the live events
+    # dominant kernel: the FP32 iterations; time per iteration from the live events (the passes
+    # that start a segment included)
     spmv_n, spmv_t, spmv_ms = tm["f32_spmv"]
-    avg_s = spmv_ms / max(spmv_t, 1) / 1e3
+    avg_s = spmv_ms / max(prof_iters, 1) / 1e3
     coef_used = bool(d_fast.inner_operator)
     algo_bytes = (F32_COEF_BYTES_PER_ROW if coef_used else F32_SPMV_BYTES_PER_ROW) * n
     peaks = {}
@@ -520,32 +522,32 @@ def run_ours(args):
     peak_note = "of measured" if hbm else "of fallback"
     hbm = hbm or 6650.0
     achieved = algo_bytes / avg_s / 1e9 if avg_s > 0 else 0.0
-    # DRAM bytes per launch of the same kernel from one ncu capture (profiles/traffic.json)
+    # DRAM bytes per iteration of the same kernel from one ncu capture (profiles/traffic.json)
     tr_all = {}
     tr_path = os.path.join(REPO, "profiles", "traffic.json")
     if os.path.exists(tr_path):
         tr_all = {k: v for k, v in json.load(open(tr_path)).items() if v.get("ne") == ne}
     tr = tr_all.get("f32_cg_coef" if coef_used else "f32_cg_band", {})
-    traffic, limiter = tr.get("bytes_per_launch"), tr.get("limiter")
+    traffic, limiter = tr.get("bytes_per_iteration"), tr.get("limiter")
     roofline = {"bound": "hbm",
-                "kernel": ("k_f32_cg<27, element coefficients> (one fused FP32 PCG iteration: operator from kappa per "
-                           "element, vector updates, one reduction)" if coef_used else
-                           "k_f32_cg<27, band> (one fused FP32 PCG iteration: 27-band SpMV, vector updates, one "
-                           "reduction)"),
+                "kernel": ("k_f32_cg_coef<3> (FP32 PCG iterations, many per launch: operator from kappa per "
+                           "element, vector updates, one grid-wide exchange each)" if coef_used else
+                           "k_f32_cg<27> (FP32 PCG iterations, many per launch: 27-band SpMV, vector updates, one "
+                           "grid-wide exchange each)"),
                 "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s",
                 "frac": round(achieved / hbm, 4), "peak_source": peak_note,
-                "algorithmic_bytes_per_launch": algo_bytes, "avg_launch_us": round(avg_s * 1e6, 2),
-                "launches_timed": spmv_t, "traffic": traffic, "limiter": limiter,
-                "timing": f"CUDA events around each launch over {n_prof} steps (graphs off: {ms_events:.1f} ms/step)"}
+                "algorithmic_bytes_per_iteration": algo_bytes, "avg_iteration_us": round(avg_s * 1e6, 2),
+                "iterations_timed": prof_iters, "launches_timed": spmv_t, "traffic": traffic, "limiter": limiter,
+                "timing": f"CUDA events around each launch over {n_prof} steps ({ms_events:.1f} ms/step)"}
 
     # the pipeline configuration the tuner chose for the timed path's operator (read before
     # another solve switches the matrix's workspace to another operator)
     cfg, ug = C.c_int(), C.c_int()
     spmv_us = (C.c_double * 2)()
     lib.rg_solver_config(mat, C.byref(cfg), C.byref(ug), spmv_us)
-    spmv_names = ({0: "k_f32_cg<27, element coefficients, 3 stages x 2 CTAs/SM>",
-                   1: "k_f32_cg<27, element coefficients, 2 stages x 2 CTAs/SM>"} if coef_used else
-                  {0: "k_f32_cg<27, band, 3 stages x 1 CTA/SM>", 1: "k_f32_cg<27, band, 2 stages x 2 CTAs/SM>"})
+    spmv_names = ({0: "k_f32_cg_coef<3, 2 lines/warp, 16 warps/CTA>",
+                   1: "k_f32_cg_coef<3, 1 line/warp, 28 warps/CTA>"} if coef_used else
+                  {0: "k_f32_cg<27, 3 stages x 1 CTA/SM>", 1: "k_f32_cg<27, 2 stages x 2 CTAs/SM>"})
     roofline["kernel"] = spmv_names.get(cfg.value, roofline["kernel"])
     roofline["tuned"] = {"spmv_config": cfg.value, "update_grid": ug.value,
                          "spmv_us_per_config": [round(v, 2) for v in spmv_us]}
@@ -644,11 +646,11 @@ def run_ours(args):
     kernels = {k: {"launches_per_step": v[0] // n_prof, "ms_per_step": round(v[2] / n_prof, 3)}
                for k, v in tm.items() if v[0]}
     band_bytes = F32_SPMV_BYTES_PER_ROW * n
-    roofline_band = {"kernel": "k_f32_cg<27, band> (the same iteration streaming the FP32 band copy)",
-                     "algorithmic_bytes_per_launch": band_bytes, "avg_launch_us": round(band_us, 2),
+    roofline_band = {"kernel": "k_f32_cg<27> (the same iterations streaming the FP32 band copy)",
+                     "algorithmic_bytes_per_iteration": band_bytes, "avg_iteration_us": round(band_us, 2),
                      "achieved": round(band_bytes / (band_us * 1e-6) / 1e9, 1), "peak": hbm, "unit": "GB/s",
                      "frac": round(band_bytes / (band_us * 1e-6) / 1e9 / hbm, 4), "peak_source": peak_note,
-                     "traffic": tr_all.get("f32_cg_band", {}).get("bytes_per_launch")}
+                     "traffic": tr_all.get("f32_cg_band", {}).get("bytes_per_iteration")}
 
     # --- batched workload: 64 Bricks with edges from {32,48,64,80,96} per axis, 8 right hand
     # sides each, FP32-inner/FP64-refinement PCG to rtol 1e-8, one batch (timed separately)
