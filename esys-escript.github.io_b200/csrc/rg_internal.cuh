@@ -91,8 +91,9 @@ constexpr int64_t kCoefPad = 1024;
 struct CoefRecord {
     int state = 0;              // 0: values are zero, 1: khat describes them, -1: not representable
     bool constrained = false;   // a constraint was recorded (a later assembly is not representable)
+    void* block = nullptr;      // the memory of the three below
     float* khat = nullptr;
-    double* khat64 = nullptr;   // the same in FP64 (paso's FP64 PCG)
+    double* khat64 = nullptr;   // the same in FP64 (paso's FP64 PCG; only where coef64_grid)
     int* bad = nullptr;         // set on the device when an element's A is not kappa I with kappa >= 0
 };
 
@@ -302,6 +303,7 @@ int coef_on_assemble(Matrix* m, const rg_coef* c[6], bool reduced);        // be
 int coef_on_constraint(Matrix* m, const double* q);                        // insertConstraint (not rhs_only)
 // whether the record describes the values (reads the device flag: synchronises the stream)
 int coef_usable(Matrix* m, bool* usable);
+bool coef64_grid(const Domain* d);  // whether paso's FP64 PCG uses khat64 on this grid (rg_solver.cu)
 void free_coef(Matrix* m);
 
 }  // namespace rg

@@ -2548,7 +2548,7 @@ int solve_impl(Matrix* m, const double* rhs, double* x, const rg_solver_opts* o,
     if (fp32 && o->layout == RG_LAYOUT_COEF && (rc = coef_usable(m, &coef))) return rc;
     if ((rc = prepare(m, fp32 && !coef, band64))) return rc;
     bool coef64 = false;
-    if (paso && o->sweeps <= 1 && d->dim == 3 && n >= kCoef64Rows && !m->values_out && (rc = coef_usable(m, &coef64))) return rc;
+    if (paso && o->sweeps <= 1 && coef64_grid(m->dom) && !m->values_out && (rc = coef_usable(m, &coef64))) return rc;
     w->coef64 = coef64;
     w->band64 = band64;
     w->coef_op = coef;
@@ -2693,5 +2693,7 @@ int solve_impl(Matrix* m, const double* rhs, double* x, const rg_solver_opts* o,
 }
 
 }  // namespace
+
+bool coef64_grid(const Domain* d) { return d->dim == 3 && d->n >= kCoef64Rows; }
 
 }  // namespace rg
