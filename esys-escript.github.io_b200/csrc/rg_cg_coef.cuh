@@ -14,9 +14,9 @@
 // state): 8 bytes every second iteration, the same roundings in the same order; a step still to be taken
 // when the iterations end (dpend) is taken where d is folded into the solution.
 //
-// What bounds it: L2 at 128^3 (68 MB of state, written and read alternately, and 17 MB of kappa and d in
-// an L2 that keeps about 70 MB of such a pattern: a copy of 50 MB runs at 6.9 TB/s, one of 34 MB at 8.1),
-// HBM at 256^3.  Measured per iteration against one launch per iteration with 27 formed coefficients per
+// What bounds it: loads from L2 and the exchange at 128^3 (issue slots 48 % active, DRAM 17 %;
+// 68 MB of state, written and read alternately, and 17 MB of kappa and d in an L2 that keeps about 70 MB of
+// such a pattern: a copy of 50 MB runs at 6.9 TB/s, one of 34 MB at 8.1), HBM at 256^3.  Measured per iteration against one launch per iteration with 27 formed coefficients per
 // row: 21.9 against 44.5 us at 128^3, 175 against 277 us at 256^3.
 #pragma once
 

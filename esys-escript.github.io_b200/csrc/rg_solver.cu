@@ -95,7 +95,7 @@ struct Workspace {
     int graph_sweeps[3] = {0, 0, 0};  // Jacobi sweeps the captured iterations apply
     long long graph_launches[3][T_COUNT] = {};
     int sweeps = 1;  // Jacobi sweeps of the current paso solve (Smoother.cpp:100-128)
-    bool band64 = false;              // paso FP64 with extra sweeps on the FP64 band copy (RG_LAYOUT_BAND)
+    bool band64 = false;              // FP64 iterations on the FP64 band copy (RG_LAYOUT_BAND)
     bool graph_band64[3] = {false, false, false};
     int spmv_cfg = -1;   // FP32 iteration pipeline of the band operator (kSpmvCfg; -1: not tuned)
     int coef_cfg = -1;   // the same for the element-coefficient operator (kCoefCfg)

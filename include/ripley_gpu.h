@@ -192,10 +192,11 @@ int rg_save_mm(rg_matrix* mat, const char* path);
 #define RG_LAYOUT_CSR 0           /* inner SpMV on the paso CSR values                       */
 #define RG_LAYOUT_BAND 1          /* SpMV on a 27-band (9 in 2D) structured copy: FP32_REFINE
                                      always; FP64 paso solves with extra Jacobi sweeps and
-                                     this layout stream an FP64 band copy.  FP64 solves with
-                                     one sweep run alike with either layout: they read the
-                                     CSR values without the column indices (8 bytes per
-                                     entry).  Scalar PDEs only: systems (block size 2, 3)
+                                     FP64 standard solves on 3D grids of 1.5 million nodes or
+                                     more stream an FP64 band copy.  Other FP64 solves run
+                                     alike with either layout, on the CSR values without the
+                                     column indices (8 bytes per entry) or, in paso mode, on
+                                     the recorded element coefficients.  Scalar PDEs only: systems (block size 2, 3)
                                      always use the block CSR                             */
 #define RG_LAYOUT_COEF 2          /* FP32_REFINE only: the FP32 inner PCG evaluates the operator
                                      from the element coefficients instead of streaming stored
