@@ -478,11 +478,11 @@ __global__ void __launch_bounds__(kAsmWarps * 32) k_assemble(const __grid_consta
         const double fl = __shfl_up_sync(0xffffffffu, f[1], 1);
         auto add = [&](auto l_) {
             constexpr int SY = decltype(l_)::value & 1, SZ = decltype(l_)::value >> 1;
+            // (element after element, as the other kernels add them: rounding then does not depend on the route)
 #pragma unroll
-            for (int c = 0; c < NK; ++c) {
-                acc[band_of<DIM>(0, SY, SZ, c)] += left[c];
-                acc[band_of<DIM>(1, SY, SZ, c)] += em[0][c];
-            }
+            for (int c = 0; c < NK; ++c) acc[band_of<DIM>(0, SY, SZ, c)] += left[c];
+#pragma unroll
+            for (int c = 0; c < NK; ++c) acc[band_of<DIM>(1, SY, SZ, c)] += em[0][c];
         };
         if (line == 0)
             add(std::integral_constant<int, 0>());
@@ -492,7 +492,8 @@ __global__ void __launch_bounds__(kAsmWarps * 32) k_assemble(const __grid_consta
             add(std::integral_constant<int, DIM == 3 ? 2 : 0>());
         else
             add(std::integral_constant<int, DIM == 3 ? 3 : 0>());
-        facc += fl + f[0];
+        facc += fl;
+        facc += f[0];
     }
     const bool owned = row && lane >= 1;
     if (owned && a.rhs) a.rhs[i] += facc;
