@@ -10,7 +10,7 @@ namespace rg {
 enum { PCG_RUN = 0, PCG_CONV = 1, PCG_MAXIT = 3, PCG_BREAK = 4, PCG_TIMEOUT = 6 };
 
 struct Pcg64State {  // (all CTAs compute the same values)
-    double alpha, beta, g1, g2, tau, tau_next, rho, delta, norm;
+    double alpha, beta, g1, g2, tau, tau_next, rho, delta, norm, norm2;
     long long iter;
     int status, stop;
 };
@@ -19,23 +19,25 @@ struct Pcg64State {  // (all CTAs compute the same values)
 // then alpha = tau / delta, breakdown on delta == 0.
 __device__ __forceinline__ void paso_after_a(Pcg64State& sc, const double* t, bool pend, double tol, long long maxit)
 {
+    // (the square root and the division, some 500 cycles each, overlap)
+    const double norm = sqrt(t[1]), tau = pend ? sc.tau_next : sc.tau, alpha = tau / t[0];
     if (pend) {
         sc.iter += 1;
-        sc.norm = sqrt(t[1]);
+        sc.norm = norm;
         if (sc.iter > maxit)
             sc.status = PCG_MAXIT;
         else if (fabs(sc.tau) <= 0.0)
             sc.status = PCG_BREAK;
         else if (sc.norm <= tol)
             sc.status = PCG_CONV;
-        sc.tau = sc.tau_next;
+        sc.tau = tau;
         if (sc.status != PCG_RUN) {
             sc.stop = 1;
             return;
         }
     }
     sc.delta = t[0];
-    sc.alpha = sc.tau / t[0];
+    sc.alpha = alpha;
     if (fabs(t[0]) <= 0.0) {  // breakFlag
         sc.iter += 1;
         sc.status = PCG_BREAK;
@@ -46,10 +48,54 @@ __device__ __forceinline__ void paso_after_a(Pcg64State& sc, const double* t, bo
 // After the update: w = {z.r, d.d, d.rs} with d = r - rs: the smoothing weights and the next beta.
 __device__ __forceinline__ void paso_after_b(Pcg64State& sc, const double* w)
 {
-    sc.g1 = fabs(w[1]) <= 0.0 ? 0.0 : -w[2] / w[1];
+    const double g = -w[2] / w[1], beta = w[0] / sc.tau;
+    sc.g1 = fabs(w[1]) <= 0.0 ? 0.0 : g;
     sc.g2 = 1.0 - sc.g1;
     sc.tau_next = w[0];
-    sc.beta = w[0] / sc.tau;
+    sc.beta = beta;
+}
+
+// k_pcg64's split of the two: the smoothing's |rs|^2 comes with phase B's sums, w = {z.r, d.d, d.rs, |rs|^2}.
+// After the product: alpha = tau / delta; a breakdown waits for the tests of the iteration before.
+__device__ __forceinline__ void paso_alpha(Pcg64State& sc, double delta, bool pend)
+{
+    sc.delta = delta;
+    sc.alpha = (pend ? sc.tau_next : sc.tau) / delta;
+    if (!pend && fabs(delta) <= 0.0) {
+        sc.iter += 1;
+        sc.status = PCG_BREAK;
+        sc.stop = 1;
+    }
+}
+
+// Called by thread 0.  (norm2: the square root, some 500 cycles, is taken only near the tolerance and at the end)
+__device__ __forceinline__ void paso_next(Pcg64State& sc, const double* w, bool pend, double tol, long long maxit)
+{
+    const double tau = pend ? sc.tau_next : sc.tau;
+    const double g = -w[2] / w[1], beta = w[0] / tau;
+    if (pend) {
+        sc.iter += 1;
+        sc.norm2 = w[3];
+        if (sc.iter > maxit)
+            sc.status = PCG_MAXIT;
+        else if (fabs(sc.tau) <= 0.0)
+            sc.status = PCG_BREAK;
+        else if (!(w[3] > 1.0000001 * (tol * tol)) && sqrt(w[3]) <= tol)
+            sc.status = PCG_CONV;
+        sc.tau = tau;
+        if (sc.status == PCG_RUN && fabs(sc.delta) <= 0.0) {
+            sc.iter += 1;
+            sc.status = PCG_BREAK;
+        }
+        if (sc.status != PCG_RUN) {
+            sc.stop = 1;
+            return;
+        }
+    }
+    sc.g1 = fabs(w[1]) <= 0.0 ? 0.0 : g;
+    sc.g2 = 1.0 - sc.g1;
+    sc.tau_next = w[0];
+    sc.beta = beta;
 }
 
 // v / d = (v m) >> (31 + s) for v < 2^31

@@ -28,11 +28,13 @@
 #include <cstdio>
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "rg_bulk.cuh"
 #include "rg_gridmail.cuh"
 #include "rg_internal.cuh"
+#include "rg_ordersum.cuh"
 #include "rg_pcg64_state.cuh"
 
 namespace rg {
@@ -95,6 +97,7 @@ struct Workspace {
     int graph_sweeps[3] = {0, 0, 0};  // Jacobi sweeps the captured iterations apply
     long long graph_launches[3][T_COUNT] = {};
     int sweeps = 1;  // Jacobi sweeps of the current paso solve (Smoother.cpp:100-128)
+    bool band_order = false;          // FP64 products summed in band order (RG_LAYOUT_BAND), not as 8 CSR lanes
     bool band64 = false;              // FP64 iterations on the FP64 band copy (RG_LAYOUT_BAND)
     bool graph_band64[3] = {false, false, false};
     int spmv_cfg = -1;   // FP32 iteration pipeline of the band operator (kSpmvCfg; -1: not tuned)
@@ -140,7 +143,7 @@ int ensure_workspace(Matrix* m, bool fp32)
             (rc = dalloc(&w->p, n)) || (rc = dalloc(&w->bb, n)) ||
             (rc = dalloc(&w->partials, (size_t)4 * kNumSMs * 64)) || (rc = dalloc(&w->counter, 1)) ||
             (rc = dalloc(&w->s, 1)) || (rc = dalloc(&w->bad, 1)) ||
-            (rc = dalloc((unsigned char**)&w->mail, kMailBytes)))
+            (rc = dalloc((unsigned char**)&w->mail, std::max(kMailBytes, kOrderBytes))))
             return rc;
         RG_CHECK_CUDA(pinned_malloc((void**)&w->hs, sizeof(Scal)));
         RG_CHECK_CUDA(pinned_malloc((void**)&w->hpoll, 2 * sizeof(Scal)));
@@ -1623,7 +1626,7 @@ constexpr int kPcgWarps = 16;
 template <int NB>
 constexpr int pcg64_stages() { return NB == 27 ? 2 : 6; }
 
-template <int NB, bool PASO>
+template <int NB, bool PASO, bool SEQ>
 int run_pcg64_t(Matrix* m, long long cap, long long* iters, int* status)
 {
     constexpr int W = kPcgWarps, S = pcg64_stages<NB>();
@@ -1633,7 +1636,7 @@ int run_pcg64_t(Matrix* m, long long cap, long long* iters, int* status)
     static std::once_flag once;
     static cudaError_t attr = cudaSuccess;
     std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(k_pcg64<NB, W, S, PASO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        attr = cudaFuncSetAttribute(k_pcg64<NB, W, S, PASO, SEQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)pcg64_smem<NB, W, S>());
     });
     RG_CHECK_CUDA(attr);
@@ -1658,23 +1661,28 @@ int run_pcg64_t(Matrix* m, long long cap, long long* iters, int* status)
     a.dinv = m->dinv;
     a.mail = w->mail;
     a.ntiles = (int)((n + 31) / 32);
-    // tiles spread evenly: rounds of the grid, then as many active warps per CTA as a round needs
-    // (with few rounds a last, nearly empty one would cost as much as a full one)
     const int sms = std::min(sm_count(), kMailCtas);
-    const int64_t rounds = (a.ntiles + (int64_t)sms * W - 1) / ((int64_t)sms * W);
-    a.wpc = (int)std::min<int64_t>(W, (a.ntiles + sms * rounds - 1) / (sms * rounds));
-    const int grid = (int)std::min<int64_t>(sms, (a.ntiles + a.wpc - 1) / a.wpc);
+    if (SEQ) {  // virtual blocks of 256 rows, one CTA per SM; a block's 8 warps are 8 chains
+        a.row_blocks = (int)std::min<int64_t>((n + kTile - 1) / kTile, sms);
+        a.tstep = 8 * a.row_blocks;
+    } else {    // of 32 rows
+        a.row_blocks = a.tstep = w->grid_rows;
+    }
+    a.chains = std::min(a.ntiles, a.tstep);
+    a.cpc = SEQ ? 8 : (a.chains + sms - 1) / sms;
+    const int grid = (a.chains + a.cpc - 1) / a.cpc;
+    a.pairs = pair_plan(n, grid);
     // about 20 ms of iterations per launch
     const double iter_s = (double)n * (8 * NB + 140) / 5.0e12 + 5e-6;
     a.max_iters = (int)std::min(std::max(0.02 / iter_s, 16.0), 8192.0);
     const int kind = PASO ? T_PASO_SPMV : T_STD_SPMV;
     long long launched = 0;
     for (;;) {
-        RG_CHECK_CUDA(cudaMemsetAsync(w->mail, 0, kMailBytes, stream()));
+        RG_CHECK_CUDA(cudaMemsetAsync(w->mail, 0, kOrderBytes, stream()));
         Scal* s = w->s;
         void* args[] = {&a, &s};
         cudaError_t e;
-        RG_TIMED(kind, (e = cudaLaunchCooperativeKernel((const void*)k_pcg64<NB, W, S, PASO>, dim3(grid),
+        RG_TIMED(kind, (e = cudaLaunchCooperativeKernel((const void*)k_pcg64<NB, W, S, PASO, SEQ>, dim3(grid),
                                                         dim3(W * 32), args, pcg64_smem<NB, W, S>(), stream())));
         RG_CHECK_CUDA(e);
         launched += a.max_iters;
@@ -1765,9 +1773,17 @@ int run_pcg64(Matrix* m, bool paso, long long cap, long long* iters, int* status
 {
     Workspace* w = m->ws;
     if (!w->p2) RG_CHECK_CUDA(dev_malloc((void**)&w->p2, sizeof(double) * m->dom->n));
-    if (m->dom->nbands == 27)
-        return paso ? run_pcg64_t<27, true>(m, cap, iters, status) : run_pcg64_t<27, false>(m, cap, iters, status);
-    return paso ? run_pcg64_t<9, true>(m, cap, iters, status) : run_pcg64_t<9, false>(m, cap, iters, status);
+    const bool seq = w->band_order;
+    auto run = [&](auto nb, auto p) {
+        constexpr int NB = decltype(nb)::value;
+        constexpr bool PASO = decltype(p)::value;
+        return seq ? run_pcg64_t<NB, PASO, true>(m, cap, iters, status)
+                   : run_pcg64_t<NB, PASO, false>(m, cap, iters, status);
+    };
+    using three = std::integral_constant<int, 27>;
+    using two = std::integral_constant<int, 9>;
+    if (m->dom->nbands == 27) return paso ? run(three(), std::true_type()) : run(three(), std::false_type());
+    return paso ? run(two(), std::true_type()) : run(two(), std::false_type());
 }
 
 // configurations of the FP32 iteration: (stages, CTAs per SM) of the pipeline on the band copy,
@@ -2551,6 +2567,7 @@ int solve_impl(Matrix* m, const double* rhs, double* x, const rg_solver_opts* o,
     if (paso && o->sweeps <= 1 && coef64_grid(m->dom) && !m->values_out && (rc = coef_usable(m, &coef64))) return rc;
     w->coef64 = coef64;
     w->band64 = band64;
+    w->band_order = !fp32 && o->layout == RG_LAYOUT_BAND;
     w->coef_op = coef;
     dg.inner_operator = coef ? 1 : 0;
     const double t_setup = now_s();
