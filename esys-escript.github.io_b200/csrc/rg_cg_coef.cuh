@@ -16,8 +16,10 @@
 //
 // What bounds it: loads from L2 and the exchange at 128^3 (issue slots 48 % active, DRAM 17 %;
 // 68 MB of state, written and read alternately, and 17 MB of kappa and d in an L2 that keeps about 70 MB of
-// such a pattern: a copy of 50 MB runs at 6.9 TB/s, one of 34 MB at 8.1), HBM at 256^3.  Measured per iteration against one launch per iteration with 27 formed coefficients per
-// row: 21.9 against 44.5 us at 128^3, 175 against 277 us at 256^3.
+// such a pattern: a copy of 50 MB runs at 6.9 TB/s, one of 34 MB at 8.1), HBM at
+// 256^3.  Measured per iteration (launches of ten) against one launch per iteration with a row's 27
+// coefficients formed and multiplied by one thread: 27.3 against 46.3 us at 128^3, 180 against 269 us at
+// 256^3, with the same bits.
 #pragma once
 
 struct CoefCgArgs {
@@ -43,7 +45,7 @@ struct CoefCgOp {
     const float4* vin;
     float4* vout;
     float* d;
-    float alpha, beta, tdiag;
+    float alpha, beta;
     float before;                     // the step length of the iteration before, when d has yet to take it
     bool step_d;                      // whether this iteration updates d
     double v[5];                      // r.u, u.w, u.s, p.w, p.s
@@ -61,10 +63,10 @@ struct CoefCgOp {
         k.pn = fmaf(beta, s.w, s.x);
         return fmaf(-alpha, k.spn, s.x);  // u_{i+1}, as next_u forms it
     }
-    __device__ __forceinline__ void emit(int row, float un, const Keep& k, float au, float ks, bool fixed)
+    __device__ __forceinline__ void emit(int row, float un, const Keep& k, float au, float dg, bool fixed)
     {
         const float w = fixed ? 0.f : au;
-        const float diag = fixed ? 1.f : tdiag * ks;
+        const float diag = fixed ? 1.f : dg;
         if (step_d) d[row] = fmaf(alpha, k.pn, k.d);
         vout[row] = make_float4(un, __fdividef(w, diag), k.spn, k.pn);
         const double du = un, dd = diag, dw = w, dp = k.pn, ds = (double)k.spn * dd;
@@ -84,7 +86,6 @@ struct CoefStartOp {
     using Keep = float4;
     const float4* vin;
     float4* vout;
-    float tdiag;
     double v[6];
     __device__ __forceinline__ Side load(int row) const { return load_ahead(vin + row); }
     __device__ __forceinline__ Center load_center(int row) const { return load_ahead(vin + row); }
@@ -94,10 +95,10 @@ struct CoefStartOp {
         k = c;
         return PASS == 0 ? c.w : c.x;
     }
-    __device__ __forceinline__ void emit(int row, float, const Keep& k, float au, float ks, bool fixed)
+    __device__ __forceinline__ void emit(int row, float, const Keep& k, float au, float dg, bool fixed)
     {
         const float w = fixed ? 0.f : au;
-        const float diag = fixed ? 1.f : tdiag * ks;
+        const float diag = fixed ? 1.f : dg;
         if (PASS == 0) {
             vout[row] = make_float4(k.x, 0.f, __fdividef(w, diag), k.w);
         } else {
@@ -131,12 +132,12 @@ __global__ void __launch_bounds__(W * 32, 1) k_f32_cg_coef(const __grid_constant
     unsigned gen = 0;
     for (int it = 0; it < a.max_iters; ++it) {
         const bool step_d = sc.dpend_on != 0;
-        CoefCgOp op{a.v[par], a.v[par ^ 1], a.d, (float)sc.alpha, (float)sc.beta, a.t.diag, (float)sc.dpend, step_d, {}};
+        CoefCgOp op{a.v[par], a.v[par ^ 1], a.d, (float)sc.alpha, (float)sc.beta, (float)sc.dpend, step_d, {}};
         if (warp < a.g.wpc)
             for (int blk = blockIdx.x; blk < a.g.per_slab * a.g.slabs; blk += gridDim.x) {
                 const int slab = blk / a.g.per_slab, strip = (blk - slab * a.g.per_slab) * a.g.wpc + warp;
                 if (strip < a.g.strips)
-                    march_task<DIM, NR, float, float>(a.g, a.t, a.khat, strip, slab, lane, op);
+                    march_task<DIM, NR, float, BandRow<DIM>>(a.g, a.t, a.khat, strip, slab, lane, op);
             }
         double t[5];
         ++gen;
@@ -173,13 +174,13 @@ __global__ void __launch_bounds__(128) k_f32_cg_coef_start(const __grid_constant
 {
     const int lane = threadIdx.x & 31;
     const int par = (int)(s->pk & 1);
-    CoefStartOp<0> op0{a.v[par], a.v[par ^ 1], a.t.diag, {}};
-    CoefStartOp<1> op1{a.v[par], a.v[par ^ 1], a.t.diag, {}};
+    CoefStartOp<0> op0{a.v[par], a.v[par ^ 1], {}};
+    CoefStartOp<1> op1{a.v[par], a.v[par ^ 1], {}};
     const int warps = (int)((gridDim.x * blockDim.x) >> 5);
     for (int task = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); task < a.g.strips * a.g.slabs; task += warps) {
         const int slab = task / a.g.strips, strip = task - slab * a.g.strips;
-        march_task<DIM, 1, float, float>(a.g, a.t, a.khat, strip, slab, lane, op0);
-        march_task<DIM, 1, float, float>(a.g, a.t, a.khat, strip, slab, lane, op1);
+        march_task<DIM, 1, float, BandRow<DIM>>(a.g, a.t, a.khat, strip, slab, lane, op0);
+        march_task<DIM, 1, float, BandRow<DIM>>(a.g, a.t, a.khat, strip, slab, lane, op1);
     }
     double tt[6];
     if (grid_reduce<6>(op1.v, rb, tt) && threadIdx.x == 0) {

@@ -9,16 +9,21 @@
 // there.  Two lines per lane share the loads, values and x-neighbours of the lines between them: 4 lines
 // for 2 rows instead of 3 for one.
 //
-// In a layer between two planes the 2^(dim-1) elements beside a node column contribute
-//   sum_e kappa_e (P_e(z) + Q_e(z+1) + w)  to the lower node,
-//   sum_e kappa_e (P_e(z+1) + Q_e(z) - w)  to the upper,
-// where P_e and Q_e are the element's in-plane differences to the node's own value, weighted with
-// the Q1 table entries of nodes in the same plane and in different planes, and w = S_Q (u(z+1) -
-// u(z)), S_Q the sum of the latter (a row of the table sums to zero).  The table weights come after the
-// sums over the elements (differences in x times kappa summed over y, and so on), so a node costs 8
-// differences and about 34 multiply-adds instead of 27 coefficients formed and multiplied; products of
-// differences also round better than products of the values.  A plane's sums with kappa below and
-// above it are formed when the plane is there, so that only their results are carried to the next.
+// Two ways to form a node's product:
+//  DiffRow (FP64).  In a layer between two planes the elements beside a node column contribute
+//     sum_e kappa_e (P_e(z) + Q_e(z+1) + w)  to the lower node,
+//     sum_e kappa_e (P_e(z+1) + Q_e(z) - w)  to the upper,
+//   where P_e and Q_e are the element's in-plane differences to the node's own value, weighted with
+//   the Q1 table entries of nodes in the same plane and in different planes, and w = S_Q (u(z+1) -
+//   u(z)), S_Q the sum of the latter (a row of the table sums to zero).  The table weights come after the
+//   sums over the elements (differences in x times kappa summed over y, and so on), so a node costs 8
+//   differences and about 34 multiply-adds instead of 27 coefficients formed and multiplied.
+//  BandRow (FP32).  The 27 (9) coefficients T (sum of kappa), and the products added in band order, as a row of
+//   the stored matrix: in FP32 another order ends a refinement elsewhere below the tolerance (1e-9 of the
+//   solution), and this one is what every configuration and the segment start return bit for bit.  A
+//   plane's values finish the node below (its upper nine), go into the node itself, and start the node above,
+//   whose lower nine coefficients are the upper nine of this one: 27.3 us
+//   per iteration at 128^3 and 180 at 256^3 against 26.8 and 178 by differences (which carry fewer terms).
 //
 // What is stored of the next plane's nodes, and kappa of the layer below it, is loaded into registers
 // before the arithmetic of a layer.  Staged in shared memory instead (per-lane cp.async, three planes
@@ -27,7 +32,7 @@
 #pragma once
 
 constexpr int kStrip = 30;            // run positions a warp owns
-constexpr int kMarchAhead = 1;        // planes loaded ahead (2 and 3 were slower: 26 and 27 against 22 us at 128^3)
+constexpr int kMarchAhead = 1;        // planes loaded ahead (by differences, 2 and 3 were slower: 26 and 27 against 22 us at 128^3)
 
 struct MarchGeom {
     int M, NN0, NL, NP;               // nodes per plane, per line; lines per plane; planes
@@ -40,29 +45,24 @@ struct MarchGeom {
 // Table entries T[x differs + 2 (y differs) + 4 (z differs)]; in 2D the marching axis is y.
 template <typename T>
 struct MarchTab {
-    T px, py, pxy;                    // same plane
+    T t[8];
+    T px, py, pxy;                    // DiffRow: same plane
     T qx, qy, qxy;                    // different planes
     T sq;                             // sum of the different-plane entries, the node's own column included
-    T diag;                           // the node itself
 };
 
 template <typename T>
-MarchTab<T> march_table(int dim, const double (&t)[8])
+MarchTab<T> march_table(const double (&t)[8])
 {
     MarchTab<T> m{};
+    for (int k = 0; k < 8; ++k) m.t[k] = (T)t[k];
     m.px = (T)t[1];
-    m.diag = (T)t[0];
-    if (dim == 3) {
-        m.py = (T)t[2];
-        m.pxy = (T)t[3];
-        m.qx = (T)t[5];
-        m.qy = (T)t[6];
-        m.qxy = (T)t[7];
-        m.sq = (T)(t[4] + t[5] + t[6] + t[7]);
-    } else {
-        m.qx = (T)t[3];
-        m.sq = (T)(t[2] + t[3]);
-    }
+    m.py = (T)t[2];
+    m.pxy = (T)t[3];
+    m.qx = (T)t[5];
+    m.qy = (T)t[6];
+    m.qxy = (T)t[7];
+    m.sq = (T)(t[4] + t[5] + t[6] + t[7]);
     return m;
 }
 
@@ -86,16 +86,111 @@ __device__ __forceinline__ double load_ahead(const double* p)
     asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
     return v;
 }
-template <typename K>
-__device__ __forceinline__ K load_kappa(const K* p) { return load_ahead(p); }
+
+// kappa of a layer's elements beside a node: [a] along x, [b] along y
+template <typename T>
+struct Layer {
+    T k[2][2];
+};
+
+template <typename T>
+struct DiffRow {
+    static constexpr bool kThree = true;  // 3D only
+    // of the node below: its value, what it has got so far; what its plane adds to this node
+    T u_lo = 0, acc = 0, up = 0;
+    // the plane's values n[y][x] around the node, the layers below and above: emit(u, A u, diagonal) of the node below
+    template <class Emit>
+    __device__ __forceinline__ void step(const MarchTab<T>& t, const T (&n)[3][3], const Layer<T>& lb, const Layer<T>& la,
+                                         Emit emit)
+    {
+        const T u = n[1][1];
+        const T x0 = n[1][0] - u, x1 = n[1][2] - u, y0 = n[0][1] - u, y1 = n[2][1] - u;
+        const T c00 = n[0][0] - u, c10 = n[0][2] - u, c01 = n[2][0] - u, c11 = n[2][2] - u;
+        auto sums = [&](const Layer<T>& l, T& sx, T& sy, T& sxy, T& ks) {
+            const T k00 = l.k[0][0], k10 = l.k[1][0], k01 = l.k[0][1], k11 = l.k[1][1];
+            const T ky0 = k00 + k10, ky1 = k01 + k11;
+            ks = ky0 + ky1;
+            sx = fma(k10 + k11, x1, (k00 + k01) * x0);
+            sy = fma(ky1, y1, ky0 * y0);
+            sxy = fma(k11, c11, fma(k01, c01, fma(k10, c10, k00 * c00)));
+        };
+        T bx, by, bxy, ksb, ax, ay, axy, ksa;
+        sums(lb, bx, by, bxy, ksb);
+        sums(la, ax, ay, axy, ksa);
+        const T qb = fma(t.qx, bx, fma(t.qy, by, t.qxy * bxy));
+        const T qa = fma(t.qx, ax, fma(t.qy, ay, t.qxy * axy));
+        const T p = fma(t.px, bx + ax, fma(t.py, by + ay, t.pxy * (bxy + axy)));
+        const T w = t.sq * ((u - u_lo) * ksb);
+        emit(u_lo, acc + (qb + w), T(0));
+        acc = p + (up - w);
+        up = qa;
+        u_lo = u;
+    }
+    // the node of the last plane, which has no layer above
+    template <class Emit>
+    __device__ __forceinline__ void last(Emit emit) { emit(u_lo, acc, T(0)); }
+};
+
+template <int DIM>
+struct BandRow {
+    static constexpr int N = DIM == 3 ? 9 : 3;
+    // of the node below: its value, its lower and middle products, its diagonal; this node's lower products
+    float u_lo = 0.f, acc = 0.f, diag_lo = 0.f, lower = 0.f;
+    // sums of kappa over the elements that a neighbour of band j of the plane shares with the node
+    __device__ __forceinline__ static void sums(const Layer<float>& l, float (&s)[N])
+    {
+        float sx[3][2];
+#pragma unroll
+        for (int b = 0; b < (DIM == 3 ? 2 : 1); ++b) {
+            sx[0][b] = l.k[0][b];
+            sx[1][b] = l.k[0][b] + l.k[1][b];
+            sx[2][b] = l.k[1][b];
+        }
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            s[x] = sx[x][0];
+            if (DIM == 3) {
+                s[(3 + x) % N] = sx[x][0] + sx[x][1];
+                s[(6 + x) % N] = sx[x][1];
+                s[x] = sx[x][0];
+            }
+        }
+    }
+    template <class Emit>
+    __device__ __forceinline__ void step(const MarchTab<float>& t, const float (&n)[3][3], const Layer<float>& lb,
+                                         const Layer<float>& la, Emit emit)
+    {
+        float sb[N], sa[N];
+        sums(lb, sb);
+        sums(la, sa);
+        float fin = acc, mid = lower, low = 0.f, diag = 0.f;
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const int x = j % 3, y = DIM == 3 ? j / 3 : 1;
+            const int cls = (x != 1) + (DIM == 3 ? 2 * (y != 1) : 0), other = cls + (DIM == 3 ? 4 : 2);
+            const float v = n[y][x];
+            fin = fmaf(t.t[other] * sb[j], v, fin);
+            const float c = t.t[cls] * (sb[j] + sa[j]);
+            mid = fmaf(c, v, mid);
+            low = fmaf(t.t[other] * sa[j], v, low);
+            if (j == N / 2) diag = c;
+        }
+        emit(u_lo, fin, diag_lo);
+        acc = mid;
+        lower = low;
+        u_lo = n[1][1];
+        diag_lo = diag;
+    }
+    template <class Emit>
+    __device__ __forceinline__ void last(Emit emit) { emit(u_lo, acc, diag_lo); }
+};
 
 // One task: strip `strip` of slab `slab`.  op.load(row) / op.load_center(row) load what is stored of a
 // node (Side / Center), op.value(side) and op.value(center, keep) form its value, keep being what emit
-// needs of a node the warp owns.  emit(row, u, keep, au, ks, fixed) gets every owned node's value,
-// (A u), the sum of kappa over its elements (the diagonal is t.diag * ks) and whether the constraint
-// fixes it (then au is meaningless).
-template <int DIM, int NR, typename T, typename K, class Op>
-__device__ __forceinline__ void march_task(const MarchGeom& g, const MarchTab<T>& t, const K* __restrict__ khat,
+// needs of a node the warp owns.  emit(row, u, keep, au, diag, fixed) gets every owned node's value,
+// (A u), the diagonal (BandRow) and whether the constraint fixes it (then au is meaningless).
+template <int DIM, int NR, typename T, class Row, class Op>
+__device__ __forceinline__ void march_task(const MarchGeom& g, const MarchTab<T>& t, const T* __restrict__ khat,
                                            int strip, int slab, int lane, Op& op)
 {
     static_assert(DIM == 3 || NR == 1, "2D marches one line");
@@ -116,11 +211,11 @@ __device__ __forceinline__ void march_task(const MarchGeom& g, const MarchTab<T>
     struct Fetched {                  // a plane's stored nodes, and kappa (a = 0) of the layer above it
         typename Op::Center rc[NR];
         typename Op::Side rs[2];
-        K k[NKL];
+        T k[NKL];
     };
-    auto fetch_kappa = [&](int z, K (&k)[NKL]) {  // of the layer below plane z
+    auto fetch_kappa = [&](int z, T (&k)[NKL]) {  // of the layer below plane z
 #pragma unroll
-        for (int l = 0; l < NKL; ++l) k[l] = load_kappa(khat + (z * g.M + ck + l * g.NN0));
+        for (int l = 0; l < NKL; ++l) k[l] = load_ahead(khat + (z * g.M + ck + l * g.NN0));
     };
     auto fetch = [&](int z, Fetched& f) {
         const int o = z * g.M;
@@ -132,26 +227,33 @@ __device__ __forceinline__ void march_task(const MarchGeom& g, const MarchTab<T>
         }
         fetch_kappa(z + 1, f.k);
     };
-    // carried from plane to plane: kappa of the layer below (with signs), and of each node its value, what
-    // it has got so far, what its plane adds to the node above, and sums of kappa
-    K kb[NKL];
-    T u_lo[NR], acc[NR], up[NR], ks_lo[NR];
+    // carried from plane to plane: kappa of the layer below, and of each node the row's sums, what emit needs
+    // of it and whether it is fixed (the sign of kappa)
+    T b0[NKL], b1[NKL];                   // of the elements at a = 0 / 1
+    Row row[NR];
     typename Op::Keep keep[NR];
-    bool fixed[NR];
+    bool fixed[NR], fixed_z[NR];
     Fetched f[kMarchAhead];
+    T kb[NKL];
     fetch_kappa(pb, kb);
 #pragma unroll
     for (int k = 0; k < kMarchAhead; ++k)
         if (pb + k <= pe) fetch(pb + k, f[k]);
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
-        u_lo[r] = acc[r] = up[r] = ks_lo[r] = T(0);
         fixed[r] = false;
+        fixed_z[r] = signbit(kb[r]);
+    }
+#pragma unroll
+    for (int l = 0; l < NKL; ++l) {
+        b0[l] = (T)fabs(kb[l]);
+        b1[l] = __shfl_down_sync(0xffffffffu, b0[l], 1);
     }
     auto plane = [&](int z, Fetched& f) {
         T v[NR + 2];
         typename Op::Keep keep_z[NR];
-        K ka[NKL];
+        T a0[NKL], a1[NKL];
+        bool fixed_a[NR];
 #pragma unroll
         for (int r = 0; r < NR; ++r) v[r + 1] = op.value(f.rc[r], keep_z[r]);
         if (DIM == 3) {
@@ -159,7 +261,9 @@ __device__ __forceinline__ void march_task(const MarchGeom& g, const MarchTab<T>
             v[NR + 1] = op.value(f.rs[1]);
         }
 #pragma unroll
-        for (int l = 0; l < NKL; ++l) ka[l] = f.k[l];
+        for (int r = 0; r < NR; ++r) fixed_a[r] = signbit(f.k[r]);
+#pragma unroll
+        for (int l = 0; l < NKL; ++l) a0[l] = (T)fabs(f.k[l]);
         if (z + kMarchAhead <= pe) fetch(z + kMarchAhead, f);
         T vl[NR + 2], vh[NR + 2];
 #pragma unroll
@@ -168,55 +272,38 @@ __device__ __forceinline__ void march_task(const MarchGeom& g, const MarchTab<T>
             vl[k] = __shfl_up_sync(0xffffffffu, v[k], 1);
             vh[k] = __shfl_down_sync(0xffffffffu, v[k], 1);
         }
-        T b0[NKL], b1[NKL], a0[NKL], a1[NKL];  // kappa below / above, of the elements at a = 0 / 1
 #pragma unroll
-        for (int l = 0; l < NKL; ++l) {
-            b0[l] = (T)fabs(kb[l]);
-            a0[l] = (T)fabs(ka[l]);
-            b1[l] = __shfl_down_sync(0xffffffffu, b0[l], 1);
-            a1[l] = __shfl_down_sync(0xffffffffu, a0[l], 1);
-        }
+        for (int l = 0; l < NKL; ++l) a1[l] = __shfl_down_sync(0xffffffffu, a0[l], 1);
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
-            const T u = v[r + 1];
-            const T x0 = vl[r + 1] - u, x1 = vh[r + 1] - u;
-            T qb, qa, p, ksb, ksa;  // the plane's sums: for the node below, for the node above, for the node
-            if (DIM == 3) {
-                const T y0 = v[r] - u, y1 = v[r + 2] - u;
-                const T c00 = vl[r] - u, c10 = vh[r] - u, c01 = vl[r + 2] - u, c11 = vh[r + 2] - u;
-                auto sums = [&](T k00, T k10, T k01, T k11, T& sx, T& sy, T& sxy, T& ks) {
-                    const T ky0 = k00 + k10, ky1 = k01 + k11;
-                    ks = ky0 + ky1;
-                    sx = fma(k10 + k11, x1, (k00 + k01) * x0);
-                    sy = fma(ky1, y1, ky0 * y0);
-                    sxy = fma(k11, c11, fma(k01, c01, fma(k10, c10, k00 * c00)));
-                };
-                T bx, by, bxy, ax, ay, axy;
-                sums(b0[r], b1[r], b0[r + 1], b1[r + 1], bx, by, bxy, ksb);
-                sums(a0[r], a1[r], a0[r + 1], a1[r + 1], ax, ay, axy, ksa);
-                qb = fma(t.qx, bx, fma(t.qy, by, t.qxy * bxy));
-                qa = fma(t.qx, ax, fma(t.qy, ay, t.qxy * axy));
-                p = fma(t.px, bx + ax, fma(t.py, by + ay, t.pxy * (bxy + axy)));
-            } else {
-                ksb = b0[0] + b1[0];
-                ksa = a0[0] + a1[0];
-                const T bx = fma(b1[0], x1, b0[0] * x0), ax = fma(a1[0], x1, a0[0] * x0);
-                qb = t.qx * bx;
-                qa = t.qx * ax;
-                p = t.px * (bx + ax);
+            T n[3][3];
+            Layer<T> lb, la;
+#pragma unroll
+            for (int y = 0; y < 3; ++y) {
+                if (DIM == 2 && y != 1) continue;
+                n[y][0] = vl[r + y];
+                n[y][1] = v[r + y];
+                n[y][2] = vh[r + y];
             }
-            const T w = t.sq * ((u - u_lo[r]) * ksb);
-            if (z > z0 && r < rows)
-                op.emit((z - 1) * g.M + c + r * g.NN0, u_lo[r], keep[r], acc[r] + (qb + w), ks_lo[r], fixed[r]);
-            acc[r] = p + (up[r] - w);
-            up[r] = qa;
-            u_lo[r] = u;
-            ks_lo[r] = ksb + ksa;
+#pragma unroll
+            for (int y = 0; y < (DIM == 3 ? 2 : 1); ++y) {
+                lb.k[0][y] = b0[r + y];
+                lb.k[1][y] = b1[r + y];
+                la.k[0][y] = a0[r + y];
+                la.k[1][y] = a1[r + y];
+            }
+            row[r].step(t, n, lb, la, [&](T u, T au, T diag) {
+                if (z > z0 && r < rows) op.emit((z - 1) * g.M + c + r * g.NN0, u, keep[r], au, diag, fixed[r]);
+            });
             keep[r] = keep_z[r];
-            fixed[r] = signbit(kb[r]);
+            fixed[r] = fixed_z[r];
+            fixed_z[r] = fixed_a[r];
         }
 #pragma unroll
-        for (int l = 0; l < NKL; ++l) kb[l] = ka[l];
+        for (int l = 0; l < NKL; ++l) {
+            b0[l] = a0[l];
+            b1[l] = a1[l];
+        }
     };
 #pragma unroll 1
     for (int z = pb; z <= pe; z += kMarchAhead) {
@@ -227,7 +314,9 @@ __device__ __forceinline__ void march_task(const MarchGeom& g, const MarchTab<T>
     if (z1 == g.NP)  // the last plane has no layer above
 #pragma unroll
         for (int r = 0; r < NR; ++r)
-            if (r < rows) op.emit((z1 - 1) * g.M + c + r * g.NN0, u_lo[r], keep[r], acc[r], ks_lo[r], fixed[r]);
+            row[r].last([&](T u, T au, T diag) {
+                if (r < rows) op.emit((z1 - 1) * g.M + c + r * g.NN0, u, keep[r], au, diag, fixed[r]);
+            });
 }
 
 // Splits the grid for `ctas` blocks of at most `warps` warps: as many slabs as make the rounds of the

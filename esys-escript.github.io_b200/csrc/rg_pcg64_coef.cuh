@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64_coef(const __grid_constant_
         if (warp < a.g.wpc)
             for (int blk = blockIdx.x; blk < blocks; blk += gridDim.x) {
                 const int slab = blk / a.g.per_slab, strip = (blk - slab * a.g.per_slab) * a.g.wpc + warp;
-                if (strip < a.g.strips) march_task<DIM, 1, double, double>(a.g, a.t, a.khat, strip, slab, lane, op);
+                if (strip < a.g.strips) march_task<DIM, 1, double, DiffRow<double>>(a.g, a.t, a.khat, strip, slab, lane, op);
             }
         double t[2];
         ++gen;

@@ -1726,7 +1726,7 @@ int run_pcg64_coef(Matrix* m, long long cap, long long* iters, int* status)
     Pcg64CoefArgs a{};
     double T[8];
     q1_table(d, T);
-    a.t = march_table<double>(d->dim, T);
+    a.t = march_table<double>(T);
     const int ctas = std::min(sm_count(), kMailCtas);
     a.g = march_geom(d->dim, d->nn, 1, ctas, W);
     a.khat = m->coef.khat64;
@@ -1976,7 +1976,7 @@ CoefCgArgs coef_cg_args(Matrix* m, int cfg)
     CoefCgArgs a{};
     double T[8];
     q1_table(d, T);
-    a.t = march_table<float>(d->dim, T);
+    a.t = march_table<float>(T);
     a.g = march_geom(d->dim, d->nn, d->dim == 3 ? kCoefLines[cfg] : 1, std::min(sm_count(), kMailCtas),
                      kCoefWarps[cfg]);
     a.khat = m->coef.khat;
