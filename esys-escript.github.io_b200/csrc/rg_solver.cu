@@ -36,6 +36,7 @@
 #include "rg_internal.cuh"
 #include "rg_ordersum.cuh"
 #include "rg_pcg64_state.cuh"
+#include "rg_ring.cuh"
 
 namespace rg {
 using namespace bulk;
@@ -1047,7 +1048,7 @@ __global__ void __launch_bounds__(kTile + 32, kCtas) k_f32_cg(const float* __res
     const WaitCtl wc = g_wait_ctl;
     const int polls = wc.polls > 0 ? wc.polls : kDefaultPolls;
     const uint64_t pol = evict_first_policy();
-    int64_t issued = 0;               // producer: tiles whose band copies were issued, over all iterations
+    RingBooks ring;                   // producer: over all iterations
     int64_t base = 0;                 // tiles of the iterations before
     unsigned gen = 0;
     bool failed = false;
@@ -1059,8 +1060,18 @@ __global__ void __launch_bounds__(kTile + 32, kCtas) k_f32_cg(const float* __res
         const bool in = interior(tile * kTile);
         mbar_expect_tx(&full[st], (uint32_t)kmat * 4u + (in ? (uint32_t)ca.nwin * wbytes : 0u));
         bulk_g2s_hint(smem + (size_t)st * stage_floats, band + (size_t)tile * NB * kTile, NB * kTile * 4, &full[st], pol);
-        issued = c + 1;
+        ring.issued = c + 1;
         return true;
+    };
+    // the state windows of the tile in that stage (none at the grid's ends, whose rows are read directly)
+    auto issue_windows = [&](int64_t c, int k, bool back, const float4* vin) {
+        const int st = (int)(c % kStages);
+        const int64_t i0 = tile_of(k, back) * kTile;
+        if (interior(i0))
+            for (int w = 0; w < ca.nwin; ++w)
+                bulk_g2s(smem + (size_t)st * stage_floats + kmat + 4 * w * ca.wlen, vin + (i0 + ca.woff[w]), wbytes,
+                         &full[st]);
+        ring.windowed = c + 1;
     };
     for (int it = 0; it < max_iters; ++it) {
         const float alpha = mode == 0 ? (float)sc.alpha : 0.f;
@@ -1076,20 +1087,17 @@ __global__ void __launch_bounds__(kTile + 32, kCtas) k_f32_cg(const float* __res
             if (lane == 0 && !wc.withhold) {
                 for (int k = 0; k < my_tiles && !failed; ++k) {
                     const int64_t c = base + k;
-                    if (issued <= c && !issue_band(c, k, odd)) {
+                    if (ring.issued <= c && !issue_band(c, k, odd)) {
                         failed = true;
                         break;
                     }
-                    const int st = (int)(c % kStages);
-                    const int64_t i0 = tile_of(k, odd) * kTile;
-                    if (interior(i0))
-                        for (int w = 0; w < ca.nwin; ++w)
-                            bulk_g2s(smem + (size_t)st * stage_floats + kmat + 4 * w * ca.wlen, vin + (i0 + ca.woff[w]),
-                                     wbytes, &full[st]);
+                    issue_windows(c, k, odd, vin);
                 }
-                if (it + 1 < max_iters)
+                if (it + 1 < max_iters && !failed) {
+                    ring.ahead(base + my_tiles, !odd);
                     for (int k = 0; k < kStages && k < my_tiles && !failed; ++k)
                         failed = !issue_band(base + my_tiles + k, k, !odd);
+                }
                 if (failed) bad = 1;
             }
         } else {
@@ -1193,24 +1201,12 @@ __global__ void __launch_bounds__(kTile + 32, kCtas) k_f32_cg(const float* __res
         base += my_tiles;
         if (sc.status == ST_TIMEOUT || (mode == 0 && sc.done)) break;
     }
-    // copies this CTA issued and nobody waited for land (bounded) before its shared memory is released: band
-    // blocks of an iteration that did not run (their windows were never issued: only the band's bytes are
-    // in flight, and the barrier stays short of them, so the wait is on the copy itself)
-    if (warp == kConsumerWarps && lane == 0 && issued > base) {
-        for (int64_t c = base; c < issued; ++c) {
-            const int st = (int)(c % kStages);
-            const int64_t i0 = tile_of((int)(c - base), (sc.pk & 1) != 0) * kTile;
-            // the windows' share of the bytes, so that the phase can complete
-            if (interior(i0))
-                for (int w = 0; w < ca.nwin; ++w)
-                    bulk_g2s(smem + (size_t)st * stage_floats + kmat + 4 * w * ca.wlen, V0 + (i0 + ca.woff[w]), wbytes,
-                             &full[st]);
-        }
-        for (int64_t c = base; c < issued; ++c)
-            for (int tries = 0; tries < (1 << 20) && !mbar_try_wait(&full[c % kStages], (uint32_t)((c / kStages) & 1));
-                 ++tries) {
-            }
-    }
+    // every copy this CTA issued lands (bounded) before its shared memory is released, whoever gave up when; band
+    // blocks of an iteration that did not run get the windows their barriers expect first
+    if (warp == kConsumerWarps && lane == 0)
+        ring.drain(
+            kStages, [&](int64_t c, int k, bool back) { issue_windows(c, k, back, V0); },
+            [&](int64_t c) { mbar_wait(&full[c % kStages], (uint32_t)((c / kStages) & 1), 1 << 20); });
     if (t == 0) {
         if (sc.status == ST_TIMEOUT)
             report_status(s, ST_TIMEOUT);
