@@ -13,7 +13,6 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
-#include <mutex>
 #include <type_traits>
 
 #include "rg_internal.cuh"
@@ -801,12 +800,8 @@ int launch_assemble(AsmArgs& a)
     constexpr int NB = DIM == 3 ? 27 : 9, kRows = kAsmRows * kAsmWarps;
     const size_t smem =
         sizeof(double) * (NQ * 8 * 4 + std::max((size_t)kRows * NB, (size_t)kAsmWarps * 32 * a.stride));
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(k_assemble<DIM, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
-    });
-    RG_CHECK_CUDA(attr);
+    static PerDevice once;
+    RG_CHECK_CUDA(raise_smem_limit(once, k_assemble<DIM, NQ>, 128 * 1024));
     const int grid = (int)((a.n + kRows - 1) / kRows);
     RG_TIMED(T_ASSEMBLE, (k_assemble<DIM, NQ><<<grid, kAsmWarps * 32, smem, stream()>>>(a)));
     RG_CHECK_LAUNCH();

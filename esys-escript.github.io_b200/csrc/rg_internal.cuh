@@ -8,6 +8,7 @@
 #include <string>
 
 #include "../../include/ripley_gpu.h"
+#include "rg_perdevice.cuh"
 
 namespace rg {
 
@@ -127,6 +128,18 @@ void dev_free(void* p);
 constexpr size_t kPinnedBlock = 1024;
 cudaError_t pinned_malloc(void** p, size_t bytes);
 void pinned_free(void* p);
+
+// lets a kernel use `bytes` of dynamic shared memory, once per device
+template <class K>
+inline cudaError_t raise_smem_limit(PerDevice& once, K* kernel, int bytes)
+{
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    return once.run(dev, cudaSuccess, [&] {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    });
+}
 
 // ---------------------------------------------------------------- deterministic reductions
 // Every block writes NV partial sums; the last block to finish (atomic ticket) sums

@@ -23,6 +23,7 @@
 // kernels queued after convergence return at once.  Elementwise kernels use 16-byte
 // vector accesses; matrix data is loaded with streaming (evict-first) hints so that the
 // solver vectors stay resident in the 126 MB L2.
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -1607,12 +1608,13 @@ int std_band_step(Matrix* m)
 
 int sm_count()
 {
-    static int count = 0;
+    static std::atomic<int> counts[kMaxDevices];
+    int dev = 0, count = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) count = counts[dev].load();
     if (!count) {
-        int dev = 0;
-        cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
         if (count <= 0) count = kNumSMs;
+        if (dev >= 0 && dev < kMaxDevices) counts[dev].store(count);
     }
     return count;
 }
@@ -1629,13 +1631,8 @@ int run_pcg64_t(Matrix* m, long long cap, long long* iters, int* status)
     Workspace* w = m->ws;
     const Domain* d = m->dom;
     const int64_t n = d->n;
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(k_pcg64<NB, W, S, PASO, SEQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)pcg64_smem<NB, W, S>());
-    });
-    RG_CHECK_CUDA(attr);
+    static PerDevice once;
+    RG_CHECK_CUDA(raise_smem_limit(once, k_pcg64<NB, W, S, PASO, SEQ>, (int)pcg64_smem<NB, W, S>()));
     Pcg64Args a{};
     a.n = (int)n;
     a.nn0 = (int)d->nn[0];
@@ -1889,27 +1886,25 @@ int cg_attribute()
 
 int tma_attributes()
 {
-    static bool done = false;
-    if (!done) {
+    static PerDevice once;
+    int dev = 0;
+    RG_CHECK_CUDA(cudaGetDevice(&dev));
+    return once.run(dev, (int)RG_OK, []() -> int {
         int rc;
         if ((rc = cg_attribute<27, 3, 1>()) || (rc = cg_attribute<27, 2, 2>()) || (rc = cg_attribute<9, 3, 1>()) ||
             (rc = cg_attribute<9, 2, 2>()))
             return rc;
-        RG_CHECK_CUDA(cudaFuncSetAttribute(k_band64_bulk<27, band64_stages<27>(), false>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)band64_smem<27, band64_stages<27>()>()));
-        RG_CHECK_CUDA(cudaFuncSetAttribute(k_band64_bulk<27, band64_stages<27>(), true>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)band64_smem<27, band64_stages<27>()>()));
-        RG_CHECK_CUDA(cudaFuncSetAttribute(k_band64_bulk<9, band64_stages<9>(), false>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)band64_smem<9, band64_stages<9>()>()));
-        RG_CHECK_CUDA(cudaFuncSetAttribute(k_band64_bulk<9, band64_stages<9>(), true>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)band64_smem<9, band64_stages<9>()>()));
-        done = true;
-    }
-    return RG_OK;
+        auto band = [](auto* kernel, size_t bytes) -> int {
+            RG_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+            return RG_OK;
+        };
+        constexpr int S3 = band64_stages<27>(), S2 = band64_stages<9>();
+        if ((rc = band(k_band64_bulk<27, S3, false>, band64_smem<27, S3>())) ||
+            (rc = band(k_band64_bulk<27, S3, true>, band64_smem<27, S3>())) ||
+            (rc = band(k_band64_bulk<9, S2, false>, band64_smem<9, S2>())))
+            return rc;
+        return band(k_band64_bulk<9, S2, true>, band64_smem<9, S2>());
+    });
 }
 
 const void* cg_kernel_for(int nb, int cfg)

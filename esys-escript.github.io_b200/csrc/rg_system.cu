@@ -15,7 +15,6 @@
 #include <cmath>
 #include <cstdio>
 #include <algorithm>
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -1067,12 +1066,8 @@ int run_pcg_sys(Matrix* m, SysWorkspace* w, long long cap)
 {
     constexpr size_t smem = sys_pcg_smem<NB, NBANDS>();
     const Domain* d = m->dom;
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(k_pcg_sys<NB, NBANDS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    });
-    RG_CHECK_CUDA(attr);
+    static PerDevice once;
+    RG_CHECK_CUDA(raise_smem_limit(once, k_pcg_sys<NB, NBANDS>, (int)smem));
     SysPcgArgs a{};
     a.n = (int)d->n;
     a.nn0 = (int)d->nn[0];

@@ -796,12 +796,8 @@ void tile_box(int W, int H, int D, int* bw, int* bh, int* bz)
 template <int COUT>
 int launch_conv3(ConvArgs& a, int ntiles)
 {
-    static bool attr = false;
-    if (!attr) {
-        RG_CHECK_CUDA(cudaFuncSetAttribute(k_conv3<COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           ConvSmem<COUT>::kBytes));
-        attr = true;
-    }
+    static PerDevice once;
+    RG_CHECK_CUDA(raise_smem_limit(once, k_conv3<COUT>, ConvSmem<COUT>::kBytes));
     RG_TIMED(T_WS_CONV, (k_conv3<COUT><<<ntiles, kConvThreads, ConvSmem<COUT>::kBytes, stream()>>>(a)));
     RG_CHECK_LAUNCH();
     return RG_OK;
@@ -810,12 +806,8 @@ int launch_conv3(ConvArgs& a, int ntiles)
 template <int COUT, int S>
 int launch_conv3_box(ConvArgs& a, int ntiles)
 {
-    static bool attr = false;
-    if (!attr) {
-        RG_CHECK_CUDA(cudaFuncSetAttribute(k_conv3_box<COUT, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           BoxSmem<COUT, S>::kBytes));
-        attr = true;
-    }
+    static PerDevice once;
+    RG_CHECK_CUDA(raise_smem_limit(once, k_conv3_box<COUT, S>, BoxSmem<COUT, S>::kBytes));
     RG_TIMED(T_WS_CONV, (k_conv3_box<COUT, S><<<ntiles, kConvThreads, BoxSmem<COUT, S>::kBytes, stream()>>>(a)));
     RG_CHECK_LAUNCH();
     return RG_OK;
@@ -860,15 +852,16 @@ int launch_conv3_boxp(ConvArgs& a, int ntiles)
     constexpr int S = kBoxPStages;
     const int bytes = BoxPSmem<COUT>::bytes(a.Cin / 16, S);
     // host-side setup once per shared-memory size (the launches of a network come back to back)
-    static int attr = 0, last_bytes = -1, slots = 0;
-    if (bytes > attr) {
+    static int attr[kMaxDevices] = {}, last_bytes = -1, slots = 0;  // (the limit per device; its slots are the same)
+    int dev = 0;
+    RG_CHECK_CUDA(cudaGetDevice(&dev));
+    if (dev >= kMaxDevices || bytes > attr[dev]) {
         RG_CHECK_CUDA(cudaFuncSetAttribute(k_conv3_boxp<COUT, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        attr = bytes;
+        if (dev < kMaxDevices) attr[dev] = bytes;
     }
     if (bytes != last_bytes) {
-        int per_sm = 0, dev = 0, sms = 0;
+        int per_sm = 0, sms = 0;
         RG_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_conv3_boxp<COUT, S>, kConvThreads, bytes));
-        RG_CHECK_CUDA(cudaGetDevice(&dev));
         RG_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         slots = std::max(per_sm, 1) * sms;
         last_bytes = bytes;
@@ -882,12 +875,8 @@ int launch_conv3_boxp(ConvArgs& a, int ntiles)
 template <int COUT>
 int launch_wgrad(WgradArgs& a, int grid)
 {
-    static bool attr = false;
-    if (!attr) {
-        RG_CHECK_CUDA(cudaFuncSetAttribute(k_wgrad<COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           WgSmem<COUT>::kBytes));
-        attr = true;
-    }
+    static PerDevice once;
+    RG_CHECK_CUDA(raise_smem_limit(once, k_wgrad<COUT>, WgSmem<COUT>::kBytes));
     RG_TIMED(T_WS_WGRAD, (k_wgrad<COUT><<<grid, kConvThreads, WgSmem<COUT>::kBytes, stream()>>>(a)));
     RG_CHECK_LAUNCH();
     return RG_OK;
