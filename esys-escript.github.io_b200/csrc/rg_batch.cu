@@ -1114,23 +1114,23 @@ int tune(Batch* b)
 void destroy(Batch* b)
 {
     if (!b) return;
-    dev_free(b->d_inst);
-    dev_free(b->d_tile_inst);
-    dev_free(b->d_units);
-    dev_free(b->d_inst_active);
-    dev_free(b->d_nactive);
-    pinned_free(b->h_nactive);
-    dev_free(b->d_rhs);
-    dev_free(b->d_cnt);
-    dev_free(b->d_part);
-    dev_free(b->p);
-    dev_free(b->q);
-    dev_free(b->r32);
-    dev_free(b->d32);
-    dev_free(b->x64);
-    dev_free(b->bb64);
-    dev_free(b->r64);
-    dev_free(b->d_user);
+    cudaFree(b->d_inst);
+    cudaFree(b->d_tile_inst);
+    cudaFree(b->d_units);
+    cudaFree(b->d_inst_active);
+    cudaFree(b->d_nactive);
+    cudaFreeHost(b->h_nactive);
+    cudaFree(b->d_rhs);
+    cudaFree(b->d_cnt);
+    cudaFree(b->d_part);
+    cudaFree(b->p);
+    cudaFree(b->q);
+    cudaFree(b->r32);
+    cudaFree(b->d32);
+    cudaFree(b->x64);
+    cudaFree(b->bb64);
+    cudaFree(b->r64);
+    cudaFree(b->d_user);
     if (b->graph) cudaGraphExecDestroy(b->graph);
     if (b->priv) cudaStreamDestroy(b->priv);
     if (b->ev_in) cudaEventDestroy(b->ev_in);
@@ -1227,7 +1227,7 @@ int rg_batch_create(rg_matrix* const* mats, int ninst, int nrhs, rg_batch** out)
     b->h_rhs.assign((size_t)ninst * b->R, Rhs{});
     cudaError_t e = cudaSuccess;
     auto A = [&](void** p, size_t bytes) {
-        if (e == cudaSuccess) e = dev_malloc(p, bytes ? bytes : 1);
+        if (e == cudaSuccess) e = cudaMalloc(p, bytes ? bytes : 1);
     };
     A((void**)&b->d_inst, sizeof(Inst) * ninst);
     A((void**)&b->d_tile_inst, sizeof(int) * b->ntiles);
@@ -1245,7 +1245,7 @@ int rg_batch_create(rg_matrix* const* mats, int ninst, int nrhs, rg_batch** out)
     A((void**)&b->bb64, sizeof(double) * nv);
     A((void**)&b->r64, sizeof(double) * nv);
     A((void**)&b->d_user, sizeof(double*) * ninst);
-    if (e == cudaSuccess) e = pinned_malloc((void**)&b->h_nactive, sizeof(int));
+    if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_nactive, sizeof(int));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->priv, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_in, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_out, cudaEventDisableTiming);

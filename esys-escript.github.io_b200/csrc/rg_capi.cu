@@ -52,18 +52,16 @@ bool coef_ok(const rg_coef* c)
 void free_domain(Domain* d)
 {
     free_domain_workspace(d);
-    {
-        Domain::Spare& sp = d->spare;
-        if (sp.val) dev_free(sp.val);
-        if (sp.bv) dev_free(sp.bv);
-        if (sp.dinv) dev_free(sp.dinv);
-        if (sp.band32) dev_free(sp.band32);
-        if (sp.dinv32) dev_free(sp.dinv32);
-        if (sp.band64) dev_free(sp.band64);
-        sp = Domain::Spare();
+    free_domain_system_workspaces(d);
+    for (Domain::Spare* sp : {&d->spare, &d->sys_spare[0], &d->sys_spare[1]}) {
+        for (void* p : {(void*)sp->val, (void*)sp->bv, (void*)sp->dinv, (void*)sp->band32, (void*)sp->dinv32, (void*)sp->band64})
+            if (p) cudaFree(p);
+        *sp = Domain::Spare();
     }
-    if (d->ptr) dev_free(d->ptr);
-    if (d->idx) dev_free(d->idx);
+    if (d->spare_coef) cudaFree(d->spare_coef);
+    d->spare_coef = nullptr;
+    if (d->ptr) cudaFree(d->ptr);
+    if (d->idx) cudaFree(d->idx);
     d->ptr = nullptr;
     d->idx = nullptr;
 }
@@ -74,10 +72,10 @@ void free_matrix(Matrix* m)
     release_workspace(m);
     free_residual_scratch(m);
     free_system_workspace(m);
-    if (m->nb == 1 && m->val) {
-        // keep the arrays for the next matrix on this domain (one set)
+    if (m->val) {
+        // keep the arrays for the next matrix of this block size on this domain (one set)
         std::lock_guard<std::mutex> lock(pool_mutex());
-        Domain::Spare& sp = m->dom->spare;
+        Domain::Spare& sp = m->nb == 1 ? m->dom->spare : m->dom->sys_spare[m->nb - 2];
         if (!sp.val) {
             sp.val = m->val;
             sp.bv = m->bv;
@@ -89,13 +87,13 @@ void free_matrix(Matrix* m)
             m->band32 = m->dinv32 = nullptr;
         }
     }
-    if (m->band64) dev_free(m->band64);
+    if (m->band64) cudaFree(m->band64);
     m->band64 = nullptr;
-    if (m->val) dev_free(m->val);
-    if (m->bv) dev_free(m->bv);
-    if (m->dinv) dev_free(m->dinv);
-    if (m->band32) dev_free(m->band32);
-    if (m->dinv32) dev_free(m->dinv32);
+    if (m->val) cudaFree(m->val);
+    if (m->bv) cudaFree(m->bv);
+    if (m->dinv) cudaFree(m->dinv);
+    if (m->band32) cudaFree(m->band32);
+    if (m->dinv32) cudaFree(m->dinv32);
     m->val = m->bv = m->dinv = nullptr;
     m->band32 = m->dinv32 = nullptr;
 }
@@ -175,8 +173,8 @@ int rg_domain_create(int dim, const int64_t ne[3], const double x0[3], const dou
     }
     build_q1_tables(dim, d.dx, &d.q1);
     build_q1_reduced_tables(dim, d.dx, &d.q1r);
-    cudaError_t e1 = dev_malloc((void**)&d.ptr, sizeof(int32_t) * (n + 1));
-    cudaError_t e2 = e1 == cudaSuccess ? dev_malloc((void**)&d.idx, sizeof(int32_t) * nnz) : e1;
+    cudaError_t e1 = cudaMalloc((void**)&d.ptr, sizeof(int32_t) * (n + 1));
+    cudaError_t e2 = e1 == cudaSuccess ? cudaMalloc((void**)&d.idx, sizeof(int32_t) * nnz) : e1;
     if (e2 != cudaSuccess) {
         free_domain(&d);
         delete h;
@@ -290,8 +288,8 @@ int rg_matrix_create(rg_domain* dom, rg_matrix** out)
     }
     cudaError_t e = cudaSuccess;
     // (two more entries: bulk copies of a run of values round its end up to 16 bytes)
-    if (!m.val) e = dev_malloc((void**)&m.val, sizeof(double) * (dom->d.nnz + 2));
-    if (e == cudaSuccess && !m.bv) e = dev_malloc((void**)&m.bv, sizeof(double) * dom->d.n);
+    if (!m.val) e = cudaMalloc((void**)&m.val, sizeof(double) * (dom->d.nnz + 2));
+    if (e == cudaSuccess && !m.bv) e = cudaMalloc((void**)&m.bv, sizeof(double) * dom->d.n);
     if (e == cudaSuccess) e = cudaMemsetAsync(m.val, 0, sizeof(double) * dom->d.nnz, stream());
     if (e != cudaSuccess) {
         free_matrix(&m);
@@ -324,8 +322,17 @@ int rg_matrix_create_system(rg_domain* dom, int block_size, rg_matrix** out)
     m.dom = &dom->d;
     m.nb = block_size;
     const size_t nv = (size_t)dom->d.nnz * block_size * block_size;
-    cudaError_t e = dev_malloc((void**)&m.val, sizeof(double) * (nv + 2));  // (as above)
-    if (e == cudaSuccess) e = dev_malloc((void**)&m.bv, sizeof(double) * dom->d.n * block_size);
+    {
+        std::lock_guard<std::mutex> lock(pool_mutex());
+        Domain::Spare& sp = dom->d.sys_spare[block_size - 2];
+        m.val = sp.val;
+        m.bv = sp.bv;
+        m.dinv = sp.dinv;
+        sp = Domain::Spare();
+    }
+    cudaError_t e = cudaSuccess;
+    if (!m.val) e = cudaMalloc((void**)&m.val, sizeof(double) * (nv + 2));  // (as above)
+    if (e == cudaSuccess && !m.bv) e = cudaMalloc((void**)&m.bv, sizeof(double) * dom->d.n * block_size);
     if (e == cudaSuccess) e = cudaMemsetAsync(m.val, 0, sizeof(double) * nv, stream());
     if (e != cudaSuccess) {
         free_matrix(&m);

@@ -12,6 +12,9 @@
 // the fixed nodes as the sign bit of khat at that node.  Anything else that changes the values
 // (B, C, D, reduced-order or face terms, nullifyRowsAndCols, an assembly after a constraint)
 // marks the record as not representable, and the solver then uses the stored values.
+#include <mutex>
+#include <utility>
+
 #include "rg_internal.cuh"
 
 namespace rg {
@@ -64,7 +67,11 @@ int coef_begin(Matrix* m)
     const size_t size = (size_t)khat_size(d), wide = coef64_grid(d) ? (sizeof(double) * size + 255) / 256 * 256 : 0;
     const size_t bytes = wide + sizeof(float) * size + sizeof(int);
     if (!c.block) {
-        RG_CHECK_CUDA(dev_malloc(&c.block, bytes));
+        {
+            std::lock_guard<std::mutex> lock(pool_mutex());
+            std::swap(c.block, m->dom->spare_coef);  // a destroyed matrix's, of the same sizes
+        }
+        if (!c.block) RG_CHECK_CUDA(cudaMalloc(&c.block, bytes));
         char* p = static_cast<char*>(c.block);
         c.khat64 = wide ? reinterpret_cast<double*>(p) : nullptr;
         c.khat = reinterpret_cast<float*>(p + wide);
@@ -144,7 +151,11 @@ int coef_usable(Matrix* m, bool* usable)
 
 void free_coef(Matrix* m)
 {
-    dev_free(m->coef.block);
+    {
+        std::lock_guard<std::mutex> lock(pool_mutex());
+        if (!m->dom->spare_coef) std::swap(m->coef.block, m->dom->spare_coef);
+    }
+    cudaFree(m->coef.block);
     m->coef = CoefRecord();
 }
 

@@ -3,6 +3,7 @@
 #include <mutex>
 
 #include <cuda_runtime.h>
+#include <initializer_list>
 #include <stdint.h>
 
 #include <string>
@@ -55,6 +56,7 @@ void build_q1_reduced_tables(int dim, const double dx[3], Q1Tables* t);
 
 // ---------------------------------------------------------------- handles
 struct Workspace;
+struct SysWorkspace;
 struct Domain {
     int dim;
     int64_t ne[3], nn[3];  // unused axes hold 1
@@ -74,6 +76,10 @@ struct Domain {
         double *val = nullptr, *bv = nullptr, *dinv = nullptr, *band64 = nullptr;
         float *band32 = nullptr, *dinv32 = nullptr;
     } spare;
+    // the same for block sizes 2 and 3 (only val, bv, dinv), their solver vectors, and a coefficient record's memory
+    Spare sys_spare[2];
+    SysWorkspace* sys_spare_ws[2] = {nullptr, nullptr};
+    void* spare_coef = nullptr;
 };
 
 struct Workspace;        // solver vectors, allocated lazily (rg_solver.cu)
@@ -120,14 +126,28 @@ struct Matrix {
     CoefRecord coef;
 };
 
-// ---------------------------------------------------------------- memory (rg_pool.cu)
-// Device blocks from the library's pool on the current device, ordered on stream(); a block is given back
-// after a device synchronisation, as cudaFree implies one.  Pinned host blocks of at most kPinnedBlock bytes.
-cudaError_t dev_malloc(void** p, size_t bytes);
-void dev_free(void* p);
-constexpr size_t kPinnedBlock = 1024;
-cudaError_t pinned_malloc(void** p, size_t bytes);
-void pinned_free(void* p);
+// ---------------------------------------------------------------- memory
+// Arrays come from cudaMalloc and go back with cudaFree, which order them against every stream, leave other
+// threads' captures alone and allow what callers do with the addresses they are handed.  What each of
+// those calls costs on a shared host (0.7 to 20 ms) is kept off the repeated path: a domain keeps one set of a
+// destroyed matrix's arrays for the next, and solver vectors are one block.
+struct BlockPart {
+    void** p;
+    size_t bytes;
+};
+inline cudaError_t alloc_block(void** block, std::initializer_list<BlockPart> parts)
+{
+    size_t total = 0;
+    for (const BlockPart& q : parts) total += (q.bytes + 255) / 256 * 256;
+    const cudaError_t e = cudaMalloc(block, total ? total : 1);
+    if (e != cudaSuccess) return e;
+    char* at = static_cast<char*>(*block);
+    for (const BlockPart& q : parts) {
+        *q.p = at;
+        at += (q.bytes + 255) / 256 * 256;
+    }
+    return e;
+}
 
 // lets a kernel use `bytes` of dynamic shared memory, once per device
 template <class K>
@@ -308,6 +328,7 @@ int launch_system_spmv(const Matrix* m, double alpha, const double* x, double be
 int solve_system(Matrix* m, const double* rhs, double* x, const rg_solver_opts* o, rg_diag* diag);
 int residual_norms_system(Matrix* m, const double* b, const double* x, double* l2, double* linf);
 void free_system_workspace(Matrix* m);
+void free_domain_system_workspaces(Domain* d);
 void free_residual_scratch(Matrix* m);
 // coefficient record of a scalar matrix (rg_coef.cu)
 void coef_reset(Matrix* m);                                                // values zeroed

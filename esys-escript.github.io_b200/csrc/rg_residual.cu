@@ -16,9 +16,9 @@ struct ResidualScratch {
 void free_residual_scratch(Matrix* m)
 {
     if (!m->rs) return;
-    dev_free(m->rs->partials);
-    dev_free(m->rs->counter);
-    dev_free(m->rs->out);
+    cudaFree(m->rs->partials);
+    cudaFree(m->rs->counter);
+    cudaFree(m->rs->out);
     delete m->rs;
     m->rs = nullptr;
 }
@@ -28,9 +28,9 @@ int ensure_residual_scratch(Matrix* m)
     if (m->rs) return RG_OK;
     ResidualScratch* s = new ResidualScratch();
     m->rs = s;
-    RG_CHECK_CUDA(dev_malloc((void**)&s->partials, sizeof(double) * residual::kMaxBlocks * 2));
-    RG_CHECK_CUDA(dev_malloc((void**)&s->counter, sizeof(unsigned)));
-    RG_CHECK_CUDA(dev_malloc((void**)&s->out, sizeof(double) * 2));
+    RG_CHECK_CUDA(cudaMalloc((void**)&s->partials, sizeof(double) * residual::kMaxBlocks * 2));
+    RG_CHECK_CUDA(cudaMalloc((void**)&s->counter, sizeof(unsigned)));
+    RG_CHECK_CUDA(cudaMalloc((void**)&s->out, sizeof(double) * 2));
     RG_CHECK_CUDA(cudaMemsetAsync(s->counter, 0, sizeof(unsigned), stream()));
     return RG_OK;
 }

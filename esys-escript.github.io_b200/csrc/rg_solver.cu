@@ -73,6 +73,7 @@ enum { ST_RUN = 0, ST_CONV = 1, ST_MAXIT = 3, ST_BREAK = 4 };
 struct Workspace {
     int64_t n = 0;
     double *r = nullptr, *x = nullptr, *rs = nullptr, *x2 = nullptr, *q = nullptr, *z = nullptr;
+    void *block = nullptr, *block32 = nullptr;  // the memory of the vectors; of the FP32 path's
     double* p = nullptr;
     double* p2 = nullptr;  // the persistent FP64 PCG's second buffer of p
     double* bvm = nullptr; // its signed balance vector when the operator is marched
@@ -111,13 +112,6 @@ struct Workspace {
 
 namespace {
 
-template <typename T>
-int dalloc(T** p, size_t count)
-{
-    RG_CHECK_CUDA(dev_malloc((void**)p, sizeof(T) * (count ? count : 1)));
-    return RG_OK;
-}
-
 int ensure_workspace(Matrix* m, bool fp32)
 {
     const int64_t n = m->dom->n;
@@ -139,28 +133,30 @@ int ensure_workspace(Matrix* m, bool fp32)
         w->n = n;
         w->grid_rows = grid_for(n, kThreads / kLpr, 8);
         w->grid_vec = grid_for((n + 3) / 4, kThreads, 8);
-        int rc;
-        if ((rc = dalloc(&w->r, n)) || (rc = dalloc(&w->x, n)) || (rc = dalloc(&w->rs, n)) ||
-            (rc = dalloc(&w->x2, n)) || (rc = dalloc(&w->q, n)) || (rc = dalloc(&w->z, n)) ||
-            (rc = dalloc(&w->p, n)) || (rc = dalloc(&w->bb, n)) ||
-            (rc = dalloc(&w->partials, (size_t)4 * kNumSMs * 64)) || (rc = dalloc(&w->counter, 1)) ||
-            (rc = dalloc(&w->s, 1)) || (rc = dalloc(&w->bad, 1)) ||
-            (rc = dalloc((unsigned char**)&w->mail, std::max(kMailBytes, kOrderBytes))))
-            return rc;
-        RG_CHECK_CUDA(pinned_malloc((void**)&w->hs, sizeof(Scal)));
-        RG_CHECK_CUDA(pinned_malloc((void**)&w->hpoll, 2 * sizeof(Scal)));
-        RG_CHECK_CUDA(cudaStreamCreateWithFlags(&w->priv, cudaStreamNonBlocking));
-        RG_CHECK_CUDA(cudaEventCreateWithFlags(&w->ev_in, cudaEventDisableTiming));
-        RG_CHECK_CUDA(cudaEventCreateWithFlags(&w->ev_out, cudaEventDisableTiming));
-        RG_CHECK_CUDA(cudaEventCreateWithFlags(&w->poll_ev[0], cudaEventDisableTiming));
-        RG_CHECK_CUDA(cudaEventCreateWithFlags(&w->poll_ev[1], cudaEventDisableTiming));
-        RG_CHECK_CUDA(cudaMemsetAsync(w->counter, 0, sizeof(unsigned), stream()));
     }
     Workspace* w = m->ws;
-    if (fp32 && !w->d32) {
-        int rc;
-        if ((rc = dalloc(&w->d32, n)) || (rc = dalloc(&w->v4[0], n)) || (rc = dalloc(&w->v4[1], n))) return rc;
+    // (a set-up that failed is taken up again by the next solve)
+    if (!w->block) {
+        const size_t v = sizeof(double) * n;
+        RG_CHECK_CUDA(alloc_block(&w->block, {{(void**)&w->r, v}, {(void**)&w->x, v}, {(void**)&w->rs, v},
+                                              {(void**)&w->x2, v}, {(void**)&w->q, v}, {(void**)&w->z, v},
+                                              {(void**)&w->p, v}, {(void**)&w->bb, v},
+                                              {(void**)&w->partials, sizeof(double) * 4 * kNumSMs * 64},
+                                              {(void**)&w->counter, sizeof(unsigned)}, {(void**)&w->s, sizeof(Scal)},
+                                              {(void**)&w->bad, sizeof(int)},
+                                              {(void**)&w->mail, std::max(kMailBytes, kOrderBytes)}}));
+        RG_CHECK_CUDA(cudaMemsetAsync(w->counter, 0, sizeof(unsigned), stream()));
     }
+    if (!w->hs) {
+        RG_CHECK_CUDA(cudaMallocHost((void**)&w->hs, 3 * sizeof(Scal)));
+        w->hpoll = w->hs + 1;
+    }
+    if (!w->priv) RG_CHECK_CUDA(cudaStreamCreateWithFlags(&w->priv, cudaStreamNonBlocking));
+    for (cudaEvent_t* e : {&w->ev_in, &w->ev_out, &w->poll_ev[0], &w->poll_ev[1]})
+        if (!*e) RG_CHECK_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    if (fp32 && !w->block32)
+        RG_CHECK_CUDA(alloc_block(&w->block32, {{(void**)&w->d32, sizeof(float) * n}, {(void**)&w->v4[0], sizeof(float4) * n},
+                                                {(void**)&w->v4[1], sizeof(float4) * n}}));
     return RG_OK;
 }
 
@@ -1710,8 +1706,8 @@ int run_pcg64_coef(Matrix* m, long long cap, long long* iters, int* status)
     Workspace* w = m->ws;
     const Domain* d = m->dom;
     const int64_t n = d->n;
-    if (!w->p2) RG_CHECK_CUDA(dev_malloc((void**)&w->p2, sizeof(double) * n));
-    if (!w->bvm) RG_CHECK_CUDA(dev_malloc((void**)&w->bvm, sizeof(double) * n));
+    if (!w->p2) RG_CHECK_CUDA(cudaMalloc((void**)&w->p2, sizeof(double) * n));
+    if (!w->bvm) RG_CHECK_CUDA(cudaMalloc((void**)&w->bvm, sizeof(double) * n));
     const int eg = grid_for(n, kThreads, 8);
     RG_TIMED(T_VECTOR, (k_pcg64_coef_enter<<<eg, kThreads, 0, stream()>>>(n, m->coef.khat64, m->bv, w->bvm, w->z, w->p,
                                                                           w->x, w->x2)));
@@ -1765,7 +1761,7 @@ int run_pcg64_coef(Matrix* m, long long cap, long long* iters, int* status)
 int run_pcg64(Matrix* m, bool paso, long long cap, long long* iters, int* status)
 {
     Workspace* w = m->ws;
-    if (!w->p2) RG_CHECK_CUDA(dev_malloc((void**)&w->p2, sizeof(double) * m->dom->n));
+    if (!w->p2) RG_CHECK_CUDA(cudaMalloc((void**)&w->p2, sizeof(double) * m->dom->n));
     const bool seq = w->band_order;
     auto run = [&](auto nb, auto p) {
         constexpr int NB = decltype(nb)::value;
@@ -2126,10 +2122,10 @@ int prepare(Matrix* m, bool want_band, bool want_band64)
     Workspace* w = m->ws;
     // a band copy is written once a solve reads it and kept current from then on; arrays
     // adopted from a destroyed matrix are not written until then
-    if (want_band && !m->band32) RG_CHECK_CUDA(dev_malloc((void**)&m->band32, sizeof(float) * d->nbands * d->npad));
-    if (want_band && !m->dinv32) RG_CHECK_CUDA(dev_malloc((void**)&m->dinv32, sizeof(float) * d->n));
+    if (want_band && !m->band32) RG_CHECK_CUDA(cudaMalloc((void**)&m->band32, sizeof(float) * d->nbands * d->npad));
+    if (want_band && !m->dinv32) RG_CHECK_CUDA(cudaMalloc((void**)&m->dinv32, sizeof(float) * d->n));
     if (want_band64 && !m->band64)
-        RG_CHECK_CUDA(dev_malloc((void**)&m->band64, sizeof(double) * d->nbands * d->npad));
+        RG_CHECK_CUDA(cudaMalloc((void**)&m->band64, sizeof(double) * d->nbands * d->npad));
     if ((want_band && !m->band32_ok) || (want_band64 && !m->band64_ok)) m->solver_ready = false;
     want_band = want_band || m->band32_ok;
     want_band64 = want_band64 || m->band64_ok;
@@ -2138,7 +2134,7 @@ int prepare(Matrix* m, bool want_band, bool want_band64)
         if (rc) return rc;
     }
     if (m->balanced && m->solver_ready) return RG_OK;
-    if (!m->dinv) RG_CHECK_CUDA(dev_malloc((void**)&m->dinv, sizeof(double) * d->n));
+    if (!m->dinv) RG_CHECK_CUDA(cudaMalloc((void**)&m->dinv, sizeof(double) * d->n));
     RG_CHECK_CUDA(cudaMemsetAsync(w->bad, 0, sizeof(int), stream()));
     int rc = launch_balance(m, m->balanced ? 0 : 1, w->bad, want_band, want_band64);
     if (rc) return rc;
@@ -2449,17 +2445,11 @@ void free_workspace(Matrix* m)
 {
     Workspace* w = m->ws;
     if (!w) return;
-    double* dd[] = {w->r, w->x, w->rs, w->x2, w->q, w->z, w->p, w->p2, w->bvm, w->bb, w->partials};
-    for (double* p : dd) dev_free(p);
-    dev_free(w->mail);
-    dev_free(w->d32);
-    dev_free(w->v4[0]);
-    dev_free(w->v4[1]);
-    dev_free(w->counter);
-    dev_free(w->s);
-    dev_free(w->bad);
-    pinned_free(w->hs);
-    pinned_free(w->hpoll);
+    cudaFree(w->block);
+    cudaFree(w->block32);
+    cudaFree(w->p2);
+    cudaFree(w->bvm);
+    cudaFreeHost(w->hs);
     for (int k = 0; k < 3; ++k)
         if (w->graph[k]) cudaGraphExecDestroy(w->graph[k]);
     if (w->ev_in) cudaEventDestroy(w->ev_in);

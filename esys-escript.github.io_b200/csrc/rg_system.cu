@@ -15,7 +15,9 @@
 #include <cmath>
 #include <cstdio>
 #include <algorithm>
+#include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "rg_bulk.cuh"
@@ -30,6 +32,7 @@ struct SysWorkspace {
     double *r = nullptr, *x = nullptr, *rs = nullptr, *x2 = nullptr, *q = nullptr, *z = nullptr,
            *p = nullptr, *p2 = nullptr, *bb = nullptr;
     unsigned long long* mail = nullptr;  // grid-wide sums of the persistent PCG (rg_gridmail.cuh)
+    void* block = nullptr;   // the memory of them all
     double* partials = nullptr;
     unsigned* counter = nullptr;
     void* s = nullptr;   // device scalars (BScal)
@@ -995,22 +998,24 @@ __global__ void __launch_bounds__(kSysWarps * 32, 1) k_pcg_sys(const __grid_cons
 // ------------------------------------------------------------------ host side
 SysWorkspace* ensure_ws(Matrix* m)
 {
-    if (m->sws) return m->sws;
-    SysWorkspace* w = new SysWorkspace();
-    const int64_t N = m->dom->n * m->nb;
-    w->N = N;
+    if (!m->sws) {
+        std::lock_guard<std::mutex> lock(pool_mutex());
+        std::swap(m->sws, m->dom->sys_spare_ws[m->nb - 2]);
+    }
+    if (!m->sws) m->sws = new SysWorkspace();
+    SysWorkspace* w = m->sws;
+    const int64_t N = w->N = m->dom->n * m->nb;
     cudaError_t e = cudaSuccess;
-    double** v[] = {&w->r, &w->x, &w->rs, &w->x2, &w->q, &w->z, &w->p, &w->p2, &w->bb};
-    for (double** pp : v)
-        if (e == cudaSuccess) e = dev_malloc((void**)pp, sizeof(double) * (N ? N : 1));
-    if (e == cudaSuccess) e = dev_malloc((void**)&w->partials, sizeof(double) * 4 * kNumSMs * 64);
-    if (e == cudaSuccess) e = dev_malloc((void**)&w->mail, kMailBytes);
-    if (e == cudaSuccess) e = dev_malloc((void**)&w->counter, sizeof(unsigned));
-    if (e == cudaSuccess) e = dev_malloc(&w->s, sizeof(BScal));
-    if (e == cudaSuccess) e = dev_malloc((void**)&w->bad, sizeof(int));
-    if (e == cudaSuccess) e = pinned_malloc(&w->hs, sizeof(BScal));
-    if (e == cudaSuccess) e = cudaMemsetAsync(w->counter, 0, sizeof(unsigned), stream());
-    m->sws = w;
+    if (!w->block) {
+        const size_t v = sizeof(double) * N;
+        e = alloc_block(&w->block, {{(void**)&w->r, v}, {(void**)&w->x, v}, {(void**)&w->rs, v}, {(void**)&w->x2, v},
+                                    {(void**)&w->q, v}, {(void**)&w->z, v}, {(void**)&w->p, v}, {(void**)&w->p2, v},
+                                    {(void**)&w->bb, v}, {(void**)&w->partials, sizeof(double) * 4 * kNumSMs * 64},
+                                    {(void**)&w->mail, kMailBytes}, {(void**)&w->counter, sizeof(unsigned)},
+                                    {&w->s, sizeof(BScal)}, {(void**)&w->bad, sizeof(int)}});
+        if (e == cudaSuccess) e = cudaMemsetAsync(w->counter, 0, sizeof(unsigned), stream());
+    }
+    if (e == cudaSuccess && !w->hs) e = cudaMallocHost(&w->hs, sizeof(BScal));
     if (e != cudaSuccess) {
         set_error(std::string("system solver workspace: ") + cudaGetErrorString(e));
         return nullptr;
@@ -1032,7 +1037,7 @@ int prepare_sys(Matrix* m, SysWorkspace* w)
 {
     const Domain* d = m->dom;
     if (m->balanced && m->solver_ready) return RG_OK;
-    if (!m->dinv) RG_CHECK_CUDA(dev_malloc((void**)&m->dinv, sizeof(double) * d->n * NB * NB));
+    if (!m->dinv) RG_CHECK_CUDA(cudaMalloc((void**)&m->dinv, sizeof(double) * d->n * NB * NB));
     const int grid = grid_for(d->n * NB, kThreads / kLpr, 16);
     if (!m->balanced) {
         RG_TIMED(T_BALANCE, (k_balance_sys<NB><<<grid, kThreads, 0, stream()>>>(d->n, d->ptr, m->val, m->bv)));
@@ -1422,19 +1427,34 @@ int solve_system(Matrix* m, const double* rhs, double* x, const rg_solver_opts* 
     return m->nb == 2 ? sys::solve_sys<2>(m, rhs, x, o, diag) : sys::solve_sys<3>(m, rhs, x, o, diag);
 }
 
+namespace {
+void free_sys(SysWorkspace* w)
+{
+    if (!w) return;
+    cudaFree(w->block);
+    cudaFreeHost(w->hs);
+    delete w;
+}
+}  // namespace
+
+// (as release_workspace: one set of vectors is kept for the next matrix of this block size)
 void free_system_workspace(Matrix* m)
 {
-    SysWorkspace* w = m->sws;
-    if (!w) return;
-    double* v[] = {w->r, w->x, w->rs, w->x2, w->q, w->z, w->p, w->p2, w->bb, w->partials};
-    for (double* p : v) dev_free(p);
-    dev_free(w->mail);
-    dev_free(w->counter);
-    dev_free(w->s);
-    dev_free(w->bad);
-    pinned_free(w->hs);
-    delete w;
+    if (!m->sws) return;
+    {
+        std::lock_guard<std::mutex> lock(pool_mutex());
+        if (!m->dom->sys_spare_ws[m->nb - 2]) std::swap(m->sws, m->dom->sys_spare_ws[m->nb - 2]);
+    }
+    free_sys(m->sws);
     m->sws = nullptr;
+}
+
+void free_domain_system_workspaces(Domain* d)
+{
+    for (SysWorkspace*& w : d->sys_spare_ws) {
+        free_sys(w);
+        w = nullptr;
+    }
 }
 
 }  // namespace rg
