@@ -9,6 +9,15 @@ namespace rg {
 // iteration status, as in the solvers' device scalars
 enum { PCG_RUN = 0, PCG_CONV = 1, PCG_MAXIT = 3, PCG_BREAK = 4, PCG_TIMEOUT = 6 };
 
+// Iterations of one launch of a persistent kernel that takes `iter_s` seconds for each: about 2 ms.  A launch holds
+// every SM, so this is how long other streams of the program wait for their turn; at 20 ms a
+// solve took 1 % less.
+inline int launch_iters(double iter_s)
+{
+    const double k = 0.002 / iter_s;
+    return k < 4.0 ? 4 : (k > 8192.0 ? 8192 : (int)k);
+}
+
 struct Pcg64State {  // (all CTAs compute the same values)
     double alpha, beta, g1, g2, tau, tau_next, rho, delta, norm, norm2;
     long long iter;

@@ -1661,9 +1661,8 @@ int run_pcg64_t(Matrix* m, long long cap, long long* iters, int* status)
     a.cpc = SEQ ? 8 : (a.chains + sms - 1) / sms;
     const int grid = (a.chains + a.cpc - 1) / a.cpc;
     a.pairs = pair_plan(n, grid);
-    // about 20 ms of iterations per launch
     const double iter_s = (double)n * (8 * NB + 140) / 5.0e12 + 5e-6;
-    a.max_iters = (int)std::min(std::max(0.02 / iter_s, 16.0), 8192.0);
+    a.max_iters = launch_iters(iter_s);
     const int kind = PASO ? T_PASO_SPMV : T_STD_SPMV;
     long long launched = 0;
     for (;;) {
@@ -1730,8 +1729,8 @@ int run_pcg64_coef(Matrix* m, long long cap, long long* iters, int* status)
     a.dinv = m->dinv;
     a.bvm = w->bvm;
     a.mail = w->mail;
-    const double iter_s = (double)n * 180 / 5.0e12 + 6e-6;  // about 20 ms of iterations per launch
-    a.max_iters = (int)std::min(std::max(0.02 / iter_s, 16.0), 8192.0);
+    const double iter_s = (double)n * 180 / 5.0e12 + 6e-6;
+    a.max_iters = launch_iters(iter_s);
     const int grid = march_ctas(a.g, ctas);
     long long launched = 0;
     for (;;) {
@@ -2017,9 +2016,8 @@ int launch_coef_start(Matrix* m, int mode)
 int run_f32(Matrix* m, int cfg, long long cap, long long* iters, int* status)
 {
     Workspace* w = m->ws;
-    // about 20 ms of iterations per launch
     const double iter_s = (double)m->dom->n * (w->coef_op ? 60 : 60 + 4 * m->dom->nbands) / 5.0e12 + 3e-6;
-    const int chunk = (int)std::min(std::max(0.02 / iter_s, 16.0), 8192.0);
+    const int chunk = launch_iters(iter_s);
     long long launched = 0;
     for (;;) {
         int rc = w->coef_op ? launch_coef(m, cfg, chunk) : launch_band_cfg(m, cfg, 0, chunk);

@@ -1100,9 +1100,8 @@ int run_pcg_sys(Matrix* m, SysWorkspace* w, long long cap)
     const int64_t rounds = (a.ntiles + (int64_t)sms * kSysWarps - 1) / ((int64_t)sms * kSysWarps);
     a.wpc = (int)std::min<int64_t>(kSysWarps, (a.ntiles + sms * rounds - 1) / (sms * rounds));
     const int grid = (int)std::min<int64_t>(sms, (a.ntiles + a.wpc - 1) / a.wpc);
-    // about 20 ms of iterations per launch
     const double iter_s = (double)d->n * (8 * NBANDS * NB * NB + 180 * NB) / 5.0e12 + 6e-6;
-    a.max_iters = (int)std::min(std::max(0.02 / iter_s, 16.0), 8192.0);
+    a.max_iters = launch_iters(iter_s);
     BScal* s = static_cast<BScal*>(w->s);
     long long launched = 0;
     for (;;) {
