@@ -20,7 +20,7 @@
 namespace rg {
 namespace {
 
-int64_t khat_size(const Domain* d) { return d->n + d->nn[0] * d->nn[1] + d->nn[0] + kCoefPad; }
+int64_t khat_size(const Domain* d) { return khat_reach(d->n, d->nn[0], d->nn[1]) + kCoefPad; }
 
 // kappa of every element from A (escript layout: A[i + dim j + dim^2 q + dim^2 Q e], Q = 2^dim
 // Gauss points when EXPANDED; PER_ELEMENT drops q; CONSTANT also drops e); *bad = 1 where A is

@@ -9,6 +9,7 @@
 #include <string>
 
 #include "../../include/ripley_gpu.h"
+#include "rg_khat.cuh"
 #include "rg_perdevice.cuh"
 
 namespace rg {
@@ -92,9 +93,8 @@ struct ResidualScratch;  // reduction scratch of rg_residual_norms (rg_residual.
 // per element (CONSTANT, PER_ELEMENT, or EXPANDED with the same value at every Gauss point)
 // and no B, C, D, followed by at most insertConstraint.  khat is node-indexed: khat[i] =
 // kappa of the element whose upper corner is node i (0 where there is no such element), with
-// the sign bit set on nodes the constraint fixes; it holds n + NN0 NN1 + NN0 + kCoefPad floats
+// the sign bit set on nodes the constraint fixes; it holds khat_reach + kCoefPad floats (rg_khat.cuh)
 // so that every element a node touches (i + {0,1} + NN0 {0,1} + NN0 NN1 {0,1}) is in range.
-constexpr int64_t kCoefPad = 1024;
 struct CoefRecord {
     int state = 0;              // 0: values are zero, 1: khat describes them, -1: not representable
     bool constrained = false;   // a constraint was recorded (a later assembly is not representable)

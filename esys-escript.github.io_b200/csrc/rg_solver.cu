@@ -1912,8 +1912,9 @@ const void* cg_kernel_for(int nb, int cfg)
 bool windows_merged(const Domain* d) { return 2 * d->nn[0] + kTile + 2 <= 3 * (kTile + 2); }
 
 // whether configuration cfg may run on this domain: on the band copy, whether it reaches its CTAs
-// per SM with this domain's windows.  On the element coefficients every grid takes configuration
-// 1; 0 is refused on 3D grids with long x-lines, which rg_solver_set_config always refused there
+// per SM with this domain's windows.  On the element coefficients every grid could take either; 0 stays refused
+// on 3D grids with x-lines longer than about a tile, because rg_solver_set_config's callers know it so (it once
+// had windows there that did not fit)
 bool cg_config_fits(const Domain* d, int cfg, bool coef)
 {
     if (coef) return cfg == 1 || d->dim == 2 || windows_merged(d);
