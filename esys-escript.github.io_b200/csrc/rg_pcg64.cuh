@@ -37,6 +37,8 @@
 struct Pcg64Args {
     int n, nn0, nn1, nn2;
     int off[27];                  // column offset of band b
+    int step[4][27];              // of a row's e-th entry from its lowest neighbour, with 3 or 2 neighbours along x (bit
+                                  // 0: 2) and y (bit 1: 2)
     unsigned m0, m1;              // row / d = (row * m) >> (31 + s) for d = nn0, nn0 nn1 (rows < 2^31)
     int s0, s1;
     const int32_t* ptr;
@@ -264,25 +266,25 @@ __global__ void __launch_bounds__(W * 32, 1) k_pcg64(const __grid_constant__ Pcg
                     }
                 }
             } else {
-                // the same entry by entry, since an entry's number says which sum it goes to: its neighbour from the
-                // node's place (shared memory holding the steps was slower: 30^3 9.0 against 8.3 us per iteration)
+                // the same entry by entry, since an entry's number says which sum it goes to: its neighbour by a
+                // table of steps
                 const int rowc = in ? row : row0;
                 const int lx = cx > 0, ly = cy > 0, lz = cz > 0;
                 const int ax = 1 + lx + (cx + 1 < (unsigned)a.nn0), ay = 1 + ly + (cy + 1 < (unsigned)a.nn1);
                 const int az = NB == 27 ? 1 + lz + (cz + 1 < (unsigned)a.nn2) : 1;
                 const int count = in ? ax * ay * az : 0;
                 const int ec = lx + ax * (ly + ay * lz);
+                const int lowest = row - lx - a.nn0 * ly - (int)plane * lz;
 #pragma unroll
                 for (int g = 0; g < NB; g += 9) {
                     double zz[9], pp[9];
 #pragma unroll
                     for (int m = 0; m < 9; ++m) {
-                        const int e = g + m;
-                        const int ey = ax == 3 ? (e * 11) >> 5 : e >> 1, kx = e - ey * ax;  // e / ax for ax = 2, 3
-                        const int kz = ay == 3 ? (ey * 11) >> 5 : ey >> 1, ky = ey - kz * ay;
-                        const int j = rowc + (kx - lx) + a.nn0 * (ky - ly) + (NB == 27 ? (int)plane * (kz - lz) : 0);
-                        zz[m] = a.z[e < count ? j : rowc];
-                        pp[m] = pold[e < count ? j : rowc];
+                        const int s3 = ay == 3 ? a.step[0][g + m] : a.step[2][g + m];
+                        const int s2 = ay == 3 ? a.step[1][g + m] : a.step[3][g + m];
+                        const int j = g + m < count ? lowest + (ax == 3 ? s3 : s2) : rowc;
+                        zz[m] = a.z[j];
+                        pp[m] = pold[j];
                     }
                     if (g == 0) waited = mbar_wait(&full[warp][st], ph, polls);
 #pragma unroll

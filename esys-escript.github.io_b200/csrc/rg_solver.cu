@@ -1635,6 +1635,9 @@ int run_pcg64_t(Matrix* m, long long cap, long long* iters, int* status)
     a.nn1 = (int)d->nn[1];
     a.nn2 = (int)d->nn[2];
     for (int b = 0; b < NB; ++b) a.off[b] = (int)d->band_off[b];
+    for (int c = 0; c < 4; ++c)
+        for (int e = 0, ax = c & 1 ? 2 : 3, ay = c & 2 ? 2 : 3; e < NB; ++e)
+            a.step[c][e] = e % ax + a.nn0 * (e / ax % ay) + (NB == 27 ? a.nn0 * a.nn1 * (e / ax / ay) : 0);
     fast_div((unsigned)a.nn0, &a.m0, &a.s0);
     fast_div((unsigned)(a.nn0 * a.nn1), &a.m1, &a.s1);
     a.ptr = d->ptr;
