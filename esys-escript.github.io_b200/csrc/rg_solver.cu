@@ -1698,9 +1698,11 @@ constexpr int kCoef64Warps = 16;
 // 500 x 420 29.6 against 22.4 ms, 1000 x 1200 269 against 246.
 constexpr int64_t kCoef64Rows = 200000;
 
-// rows of a 3D grid from which RG_LAYOUT_BAND's textbook PCG runs on the band copy, a kernel per step (whole
-// solve, against k_pcg64): 96^3 (912,673 rows) 33.0 against 30.4 ms, 128^3 (2.15 million) 87.6 against 90.3
-constexpr int64_t kBand64Rows = 1500000;
+// Rows of a 3D grid from which RG_LAYOUT_BAND's PCG runs on the band copy, a kernel per step, with the same bits:
+// its bulk-copied windows then outweigh the launches.  us per iteration against k_pcg64: textbook 70^3 (357,911
+// rows) 25.8 against 25.4, 80^3 34.5 against 35.9, 110^3 71.7 against 79.9; paso 95 x 97 x 96 (903,168) 62.9
+// against 60.5, 110^3 85.8 against 91.6, 128^3 134 against 143.
+constexpr int64_t kBand64Rows = 450000, kBand64PasoRows = 1100000;
 
 int run_pcg64_coef(Matrix* m, long long cap, long long* iters, int* status)
 {
@@ -2252,7 +2254,7 @@ int solve_fp64(Matrix* m, const rg_solver_opts* o, bool paso, OuterState& st, rg
             jacobi_sweeps(m, w->r, w->z, w->q, w->p, 2);  // the first v = prec(r): p and tau
             RG_CHECK_LAUNCH();
             // more than one Jacobi sweep has an SpMV inside the preconditioner: one kernel per step
-            rc = w->sweeps > 1 ? run_until_done(m, 0, paso_step, chunk, cnt, &it, &dst)
+            rc = w->sweeps > 1 || w->band64 ? run_until_done(m, 0, paso_step, chunk, cnt, &it, &dst)
                  : w->coef64   ? run_pcg64_coef(m, cnt, &it, &dst)
                                : run_pcg64(m, true, cnt, &it, &dst);
             if (rc) return rc;
@@ -2531,11 +2533,6 @@ int solve_impl(Matrix* m, const double* rhs, double* x, const rg_solver_opts* o,
     // every grid reduction leaves the counter at zero; clearing it here as well keeps one
     // solve independent of anything an earlier, interrupted one left behind
     RG_CHECK_CUDA(cudaMemsetAsync(w->counter, 0, sizeof(unsigned), stream()));
-    // the FP64 band copy serves the extra Jacobi sweeps, and the textbook PCG where its bulk-copied tiles
-    // outweigh the launches (kBand64Rows); else one sweep streams the CSR values without their column
-    // indices, the same bytes
-    const bool band64 = !fp32 && o->layout == RG_LAYOUT_BAND &&
-                        (paso ? o->sweeps > 1 : m->dom->dim == 3 && m->dom->n >= kBand64Rows);
     if (!fp32 && o->layout == RG_LAYOUT_COEF) {
         set_error("solver: RG_LAYOUT_COEF evaluates the FP32 inner operator; FP64 solves use RG_LAYOUT_CSR or "
                   "RG_LAYOUT_BAND");
@@ -2545,9 +2542,13 @@ int solve_impl(Matrix* m, const double* rhs, double* x, const rg_solver_opts* o,
     // when the matrix's values are what the coefficient record describes; else the band copy
     bool coef = false;
     if (fp32 && o->layout == RG_LAYOUT_COEF && (rc = coef_usable(m, &coef))) return rc;
-    if ((rc = prepare(m, fp32 && !coef, band64))) return rc;
     bool coef64 = false;
     if (paso && o->sweeps <= 1 && coef64_grid(m->dom) && !m->values_out && (rc = coef_usable(m, &coef64))) return rc;
+    // the FP64 band copy serves the extra Jacobi sweeps, and one sweep or the textbook PCG on large 3D grids; else
+    // iterations stream the CSR values without their column indices, the same bytes
+    const bool band64 = !fp32 && !coef64 && o->layout == RG_LAYOUT_BAND &&
+                        (o->sweeps > 1 || (m->dom->dim == 3 && m->dom->n >= (paso ? kBand64PasoRows : kBand64Rows)));
+    if ((rc = prepare(m, fp32 && !coef, band64))) return rc;
     w->coef64 = coef64;
     w->band64 = band64;
     w->band_order = !fp32 && o->layout == RG_LAYOUT_BAND;

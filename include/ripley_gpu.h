@@ -191,13 +191,15 @@ int rg_save_mm(rg_matrix* mat, const char* path);
 #define RG_PREC_FP32_REFINE 1     /* FP32 inner PCG, FP64 residual/update/stop test         */
 #define RG_LAYOUT_CSR 0           /* inner SpMV on the paso CSR values                       */
 #define RG_LAYOUT_BAND 1          /* SpMV on a 27-band (9 in 2D) structured copy: FP32_REFINE
-                                     always; FP64 paso solves with extra Jacobi sweeps and
-                                     FP64 standard solves on 3D grids of 1.5 million nodes or
-                                     more stream an FP64 band copy.  Other FP64 solves run
-                                     alike with either layout, on the CSR values without the
-                                     column indices (8 bytes per entry) or, in paso mode, on
-                                     the recorded element coefficients.  Scalar PDEs only: systems (block size 2, 3)
-                                     always use the block CSR                             */
+                                     always; FP64 paso solves with extra Jacobi sweeps, and
+                                     FP64 solves on large 3D grids (paso from 1.1 million
+                                     nodes, standard from 450,000) stream an FP64 band copy.
+                                     Other FP64 solves read the CSR values without the column
+                                     indices (8 bytes per entry) or, in paso mode, the
+                                     recorded element coefficients; a row's products are
+                                     added in band order with this layout, like 8 lanes on
+                                     the CSR entries with RG_LAYOUT_CSR.  Scalar PDEs only:
+                                     systems (block size 2, 3) always use the block CSR   */
 #define RG_LAYOUT_COEF 2          /* FP32_REFINE only: the FP32 inner PCG evaluates the operator
                                      from the element coefficients instead of streaming stored
                                      values (4 bytes per row instead of 108), when the matrix's

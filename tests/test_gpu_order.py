@@ -4,7 +4,8 @@ kernels therefore add as the kernel-per-step solver (and the element-by-element 
 these systems golden/order.json records: the SHA-256 of the solution's bytes and the iterations.  So does FP32 refinement on the element coefficients, whose
 products go in band order, in either configuration.  Sizes: below and
 above a 32-row tile, one and several tiles per virtual block, odd node counts, pairs beyond one pass, and
-an elongated Robin-like Brick on which another order ended 6e-10 away."""
+an elongated Robin-like Brick on which another order ended 6e-10 away; the two largest
+Bricks are where RG_LAYOUT_BAND's solves turn to the band copy."""
 import hashlib
 import json
 import os
@@ -21,7 +22,7 @@ pytestmark = pytest.mark.gpu
 
 GOLDEN = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden", "order.json")
 SIZES = [(31, 1), (30, 2), (200, 200), (255, 160), (700, 699), (1100, 1150), (1, 30, 2), (6, 5, 4), (22, 28, 114),
-         (57, 54, 60)]
+         (57, 54, 60), (80, 79, 82), (104, 103, 102)]
 ROUTES = {"paso_csr": (L.RG_MODE_PASO, L.RG_LAYOUT_CSR), "paso_band": (L.RG_MODE_PASO, L.RG_LAYOUT_BAND),
           "textbook_csr": (L.RG_MODE_STANDARD, L.RG_LAYOUT_CSR), "textbook_band": (L.RG_MODE_STANDARD, L.RG_LAYOUT_BAND)}
 REFINED = [(3, 2, 5), (29, 2, 3), (30, 3, 4), (61, 1, 6), (59, 60, 2), (70, 41, 33), (46, 101, 79), (29, 4), (30, 31),
