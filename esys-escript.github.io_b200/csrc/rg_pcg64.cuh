@@ -29,7 +29,7 @@
 // What bounds it: HBM at large sizes (216 B of matrix and about 16 vector accesses of 8 B per row and iteration),
 // the two exchanges at small ones (some 4,500 of 7,000 cycles each, with the chains of dependent FP64 additions).
 // Measured per iteration against a kernel per step replayed from CUDA graphs: paso on Rectangle 200 x 200 7.4
-// against 20.2 us, Brick 21 x 17 x 14 9.5 against 13.2, 95 x 97 x 96 66 against 90, 128^3 160 against 210;
+// against 20.2 us, Brick 21 x 17 x 14 9.0 against 13.2, 95 x 97 x 96 67 against 90, 128^3 158 against 210;
 // textbook on 403 x 297 8.4 against 14.9.  (Added in an order of its own, with phase B on the tiles' rows and no
 // memory order after phase A: 5.6, 6.3, 47, 134 and 6.5 us.)
 #pragma once

@@ -13,7 +13,7 @@
 //
 // Two phases and exchanges per iteration as in k_pcg64.  Phase B goes over the rows the block's own warps
 // marched, so what it reads was written by this block.  Bound by HBM at 128^3 (19 vector accesses of 8 B
-// per row): 84 against 130 us per iteration on the CSR values.
+// per row): 84 against 158 us per iteration on the CSR values.
 #pragma once
 
 struct Pcg64CoefArgs {

@@ -1692,10 +1692,11 @@ int run_pcg64_t(Matrix* m, long long cap, long long* iters, int* status)
 
 // paso's FP64 PCG on the element coefficients, from k_paso_init's state until the device flags done
 constexpr int kCoef64Warps = 16;
-// rows of a 3D grid from which the marched operator is used.  Against the CSR values (whole solve): 48 x 50
-// x 52 (137,000 rows) 3.93 against 3.77 ms, 64^3 (275,000) 6.71 against 8.56, 80 x 70 x 90 11.7 against
-// 19.1, 128^3 75.9 against 116.9.  In 2D a row has 72 bytes of matrix and three planes of halo to march:
-// 500 x 420 29.6 against 22.4 ms, 1000 x 1200 269 against 246.
+// Rows of a 3D grid from which the marched operator is used.  Against the CSR values (whole solve, k_pcg64 with
+// sums in an order of its own): 48 x 50 x 52 (137,000 rows) 3.93 against 3.77 ms, 64^3 (275,000) 6.71 against 8.56, 80 x 70
+// x 90 11.7 against 19.1, 128^3 75.9 against 116.9.  k_pcg64 takes about a third more now, but the line stays: below
+// it solutions are bit for bit those of a kernel per step.  In 2D a row has 72 bytes of matrix and three planes of
+// halo to march: 500 x 420 29.6 against 22.4 ms, 1000 x 1200 269 against 246.
 constexpr int64_t kCoef64Rows = 200000;
 
 // Rows of a 3D grid from which RG_LAYOUT_BAND's PCG runs on the band copy, a kernel per step, with the same bits:

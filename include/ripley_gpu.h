@@ -255,7 +255,8 @@ typedef struct {
 
 void rg_solver_opts_default(rg_solver_opts* opts);
 /* setToSolution: x (n doubles) = A^-1 rhs.  rhs is not modified.  The matrix is
-   balanced in place on the first solve, as paso does; later solves reuse it. */
+   balanced in place on the first solve, as paso does; later solves reuse it.  The iterations run
+   in launches of about 2 ms that occupy the whole GPU: work on other streams waits that long. */
 int rg_solve(rg_matrix* mat, const double* rhs, double* x, const rg_solver_opts* opts,
              rg_diag* diag);
 
